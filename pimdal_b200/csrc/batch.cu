@@ -118,7 +118,7 @@ extern "C" int pimdal_group_batch_create(pimdal_ctx_t *ctx, const pimdal_aggr_ar
     g.flip = a.key_dtype == PIMDAL_I32 ? 0x80000000u : 0u;
     const uint64_t expect = std::max<uint64_t>(
         1, a.expected_groups ? a.expected_groups : std::min<uint64_t>(a.size, 1ull << 22));
-    pd_gb_mode(expect, &g.mode, &g.wrep);
+    g.mode = pd_gb_mode(expect);
     const uint64_t slots = std::max<uint64_t>(256, pd_ceil_div(expect * 100, lf));
     if (slots >= (1ull << 31)) return PIMDAL_ERR_ARG;
     g.slots = (uint32_t)slots;

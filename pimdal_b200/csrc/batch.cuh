@@ -18,9 +18,9 @@ struct pd_gb_inst {
   uint64_t *d_count;   // results[i].t_count
   uint64_t slot0;      // first slot of its table in the plan's global table
   uint32_t slots;      // table slots
-  uint32_t mode;       // shared-table mode (warp tables, CTA table, direct)
-  uint32_t wrep;       // warp-table replicas
+  uint32_t mode;       // shared-table mode (lane accumulators, CTA table, direct)
   uint32_t flip;       // 0x80000000 for signed keys (ascending output order)
+  uint32_t pad;
 };
 
 struct pd_gb_batch {
@@ -79,9 +79,9 @@ struct pd_hj_batch {
 int pd_gb_batch_run(pimdal_ctx *ctx, const pd_gb_batch &b, cudaStream_t s);
 int pd_hj_batch_run(pimdal_ctx *ctx, const pd_hj_batch &b, cudaStream_t s);
 size_t pd_gb_batch_shared_bytes();
-// Shared-table mode and replicas for an expected group count (same rule as
-// the plain hash group-by).
-void pd_gb_mode(uint64_t expected, uint32_t *mode, uint32_t *wrep);
+// Shared-table mode for an expected group count (same rule as the plain hash
+// group-by).
+uint32_t pd_gb_mode(uint64_t expected);
 // Probe tile rows of the hash join; log2 of the slots of its table for nb
 // build rows at a load factor (same rule as pimdal_hash_join).
 uint32_t pd_hj_tile_rows();

@@ -18,11 +18,11 @@
 // {count << 32 | key, sum, min, max}: the claiming compare-and-swap carries
 // the first rows' count, and every later update of the group touches the same
 // sector.  Three aggregation modes, chosen from the expected group count:
-//  - GB_WARP (a few dozen groups): each warp owns a private shared-memory
-//    table of 192 slots (split in up to 4 replicas, each for a subset of the
-//    lanes), so only a few lanes of one warp ever contend;
+//  - GB_LANE (up to 128 groups): the CTA has one shared table of 212 keys and
+//    each key 32 accumulators, one per lane number, interleaved so that a
+//    warp's updates fall in 32 different banks whatever keys its lanes hold;
 //  - GB_SMEM (up to a few thousand groups): every row updates the CTA's
-//    shared-memory table (6144 slots, 192 KB, one 1024-thread CTA per SM);
+//    shared-memory table (6784 slots, 212 KB, one 1024-thread CTA per SM);
 //  - GB_PART (many groups): the rows (key and value) are first radix-
 //    partitioned by the top bits of a multiplicative hash of the key, in
 //    stable passes of at most 6 bits, into 2^b partitions of about 1024
@@ -38,7 +38,16 @@
 //    the table is larger than an L2 budget it can be split into K sub-tables
 //    by the high hash bits and aggregated in K launches, each touching an
 //    L2-sized sub-table (PIMDAL_GROUP_L2_BUDGET_MB; one pass by default).
-// Shared tables probe 4-slot buckets of 32-bit keys with one 16-byte load.
+// The aggregation is bound by shared memory, so its cycles per row decide: 64-bit
+// sums are two 32-bit words (native adds; a 64-bit add is a compare-and-swap
+// loop), keys sit in 4-slot buckets read by one 16-byte load, a key has two
+// buckets (walking over full neighbours cost more than everything else at
+// 4096 groups), and the next rows are loaded while the current ones are
+// aggregated.  Kernel time over 2^28 rows, before and after: 16 groups 2.03 ->
+// 0.85 ms, 100 groups 4.66 -> 1.16, 1000 groups 2.47 -> 1.36, 4096 groups
+// 3.24 -> 1.44; the chunks of 2^22 groups 3.86 -> 2.93.  The line between the
+// modes at 128 groups: 100 groups take 1.16 ms with lane accumulators, 130
+// groups 1.39 ms in the CTA table.
 // A row whose group finds no shared slot within 16 buckets goes to the global
 // table; shared tables are merged into the global table at the end of each
 // CTA.  A global update reads the slot's sector once (two 16-byte loads
@@ -57,14 +66,14 @@ namespace {
 
 constexpr int GB_THREADS = 1024;
 constexpr int GB_WARPS = GB_THREADS / 32;
-constexpr uint32_t GB_SMEM_SLOTS = 6144;
-constexpr uint32_t GB_WARP_SLOTS = GB_SMEM_SLOTS / GB_WARPS;  // 192 per warp
+constexpr uint32_t GB_SMEM_SLOTS = 6784;  // 34 B each (with the claim list) fill the 227 KB of an SM
+constexpr uint32_t GB_LANE_SLOTS = GB_SMEM_SLOTS / 32;  // 212 keys with 32 accumulators each
 constexpr uint32_t GB_SMEM_PROBES = 16;  // buckets
-constexpr size_t GB_SMEM_BYTES = 32ull * GB_SMEM_SLOTS;      // 192 KB
-constexpr uint64_t GB_WARP_MAX_GROUPS = 64;                  // GB_WARP at or below
-constexpr uint64_t GB_SMEM_MAX_GROUPS = 4608;                // GB_SMEM at or below (load 3/4)
+constexpr size_t GB_SMEM_BYTES = 32ull * GB_SMEM_SLOTS;      // 212 KB
+constexpr uint64_t GB_LANE_MAX_GROUPS = 128;                 // GB_LANE at or below (load 3/5)
+constexpr uint64_t GB_SMEM_MAX_GROUPS = 4608;                // GB_SMEM at or below (load 2/3)
 constexpr uint64_t GB_L2_BUDGET = 1ull << 40;                // one pass unless overridden
-enum { GB_WARP = 0, GB_SMEM = 1, GB_DIRECT = 2, GB_PART = 3 };
+enum { GB_LANE = 0, GB_SMEM = 1, GB_DIRECT = 2, GB_PART = 3 };
 constexpr uint64_t GB_PART_GROUPS = 1024;   // groups per hash partition
 constexpr uint32_t GB_PART_MAX_BITS = 12;
 
@@ -76,7 +85,6 @@ struct GbParams {
   // global table: npasses sub-tables of sub_cap 32-byte slots
   unsigned long long *gtab;
   uint32_t sub_cap, npasses;
-  uint32_t wrep;       // GB_WARP: private replicas per warp (1, 2 or 4)
   unsigned long long *ngroups;  // compacted group count (device)
   uint32_t *ckey, *cslot;
   uint32_t *d_error;
@@ -150,38 +158,97 @@ constexpr uint32_t GB_EMPTY = 0xFFFFFFFFu;
 struct SmemTable {
   uint32_t *key;
   uint32_t *cnt;
-  long long *sum;
-  longlong2 *mm;     // (min, max)
+  uint32_t *slo, *shi;  // low and high words of the sums
+  longlong2 *mm;        // (min, max)
   uint16_t *list;    // batched runs: slots claimed since the last flush
   uint32_t *nlist;
 };
+
+// Shared-memory hash of a key (multiply and xor-shift): unrelated to the
+// multiplicative hash that partitions the rows, so that the keys of one
+// partition spread over the whole table, and cheaper than the 64-bit mix of
+// the global table's slots.  A key has two buckets, both cut from this hash.
+__device__ __forceinline__ uint32_t gb_mix32(uint32_t key) {
+  uint32_t x = (key ^ (key >> 16)) * 0x9E3779B1u;
+  x = (x ^ (x >> 15)) * 0x85EBCA77u;
+  return x ^ (x >> 13);
+}
+__device__ __forceinline__ uint32_t gb_bucket1(uint32_t x, uint32_t nb) { return __umulhi(x, nb); }
+__device__ __forceinline__ uint32_t gb_bucket2(uint32_t x, uint32_t nb) {
+  return __umulhi(x * 0xC2B2AE3Du, nb);
+}
+
+// Adds v to a 64-bit shared sum held as two words.  Shared memory adds 32-bit
+// words natively but 64-bit ones in a compare-and-swap loop.  The low words'
+// additions wrap exactly once per carry, and the addition that wraps passes
+// its carry on, so the sum is exact mod 2^64 in any order.
+__device__ __forceinline__ void smem_add64(uint32_t *lo, uint32_t *hi, unsigned long long v) {
+  const uint32_t l = (uint32_t)v;
+  const uint32_t old = atomicAdd(lo, l);
+  const uint32_t h = (uint32_t)(v >> 32) + (uint32_t)(old + l < l);
+  if (h) atomicAdd(hi, h);
+}
 
 __device__ __forceinline__ int bucket_match(const uint4 &q, uint32_t key) {
   return q.x == key ? 0 : q.y == key ? 1 : q.z == key ? 2 : q.w == key ? 3 : -1;
 }
 
-// Slot of `key` in buckets [base, base + nb) of a shared table, claiming an
-// empty slot when the key is absent; -1 when no bucket within the probe limit
-// has room (the row then goes to the global table).
-__device__ __noinline__ int smem_find(const SmemTable &t, uint32_t base, uint32_t nb, uint32_t key,
-                                      uint32_t b) {
+// Occupied entries of a bucket (they are claimed in order, so they form a prefix).
+__device__ __forceinline__ int bucket_used(const uint4 &q) {
+  return q.w != GB_EMPTY ? 4 : q.z != GB_EMPTY ? 3 : q.y != GB_EMPTY ? 2 : q.x != GB_EMPTY ? 1 : 0;
+}
+
+// Slot of `key` in the nb buckets of a shared table, claiming an empty slot
+// when the key is absent; -1 when no bucket within the probe limit has room
+// (the row then goes to the global table).  The first bucket takes keys until
+// it holds two; later ones go to the emptier of the two buckets, and a key
+// that finds both full walks on from the second.  At 4096 keys in 1696
+// buckets 0.07% of the keys walk, against 6% when full buckets overflow into
+// their neighbours (3.3 ms per 2^28 rows, the walks dominating).  Two lanes
+// may claim a key in both of its buckets at once; each then collects a part
+// of the group's rows and the merge into the global table adds them up.
+// (The table's fields are passed by value: a reference would make every caller
+// keep the struct in local memory.)
+__device__ __noinline__ int smem_find(uint32_t *tkey, uint16_t *list, uint32_t *nlist, uint32_t nb,
+                                      uint32_t key) {
+  const uint32_t x = gb_mix32(key);
+  const uint32_t b1 = gb_bucket1(x, nb), b2 = gb_bucket2(x, nb);
+  uint32_t b = b1;
   for (uint32_t i = 0; i < GB_SMEM_PROBES;) {
-    const uint32_t s0 = 4 * (base + b);
     // plain loads: a key never changes once set, so a stale bucket costs at
     // most a failed compare-and-swap and another look
-    const uint4 q = *reinterpret_cast<const uint4 *>(t.key + s0);
-    const int hit = bucket_match(q, key);
-    if (hit >= 0) return (int)s0 + hit;
-    const int e = bucket_match(q, GB_EMPTY);
-    if (e < 0) {  // full bucket without the key: next bucket
+    uint4 q;
+    if (i == 0) {
+      const uint4 q1 = *reinterpret_cast<const uint4 *>(tkey + 4 * b1);
+      const uint4 q2 = *reinterpret_cast<const uint4 *>(tkey + 4 * b2);
+      const int h1 = bucket_match(q1, key), h2 = bucket_match(q2, key);
+      if (h1 >= 0) return (int)(4 * b1) + h1;
+      if (h2 >= 0) return (int)(4 * b2) + h2;
+      const int n1 = bucket_used(q1), n2 = bucket_used(q2);
+      if (n1 >= 2 && n2 < n1) {
+        b = b2;
+        q = q2;
+      } else {
+        b = b1;
+        q = q1;
+      }
+    } else {
+      q = *reinterpret_cast<const uint4 *>(tkey + 4 * b);
+      const int hit = bucket_match(q, key);
+      if (hit >= 0) return (int)(4 * b) + hit;
+    }
+    const int e = bucket_used(q);
+    if (e == 4) {  // full without the key: walk on from the second bucket
+      if (i == 0) b = b2;
       b = (b + 1 == nb) ? 0 : b + 1;
       ++i;
       continue;
     }
-    const uint32_t old = atomicCAS(t.key + s0 + e, GB_EMPTY, key);
-    if (old == GB_EMPTY && t.list) t.list[atomicAdd(t.nlist, 1u)] = (uint16_t)(s0 + e);
-    if (old == GB_EMPTY || old == key) return (int)s0 + e;
-    // lost the slot to another key: look at the bucket again
+    const uint32_t s = 4 * b + e;
+    const uint32_t old = atomicCAS(tkey + s, GB_EMPTY, key);
+    if (old == GB_EMPTY && list) list[atomicAdd(nlist, 1u)] = (uint16_t)s;
+    if (old == GB_EMPTY || old == key) return (int)s;
+    // lost the slot to another key: look again
   }
   return -1;
 }
@@ -192,7 +259,7 @@ __device__ __noinline__ int smem_find(const SmemTable &t, uint32_t base, uint32_
 template <int MODE>
 __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, uint32_t pass,
                                          const uint32_t (&k)[4], const long long (&v)[4],
-                                         uint32_t valid, uint32_t base, uint32_t nb) {
+                                         uint32_t valid, uint32_t nb) {
   if constexpr (MODE == GB_DIRECT) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -202,47 +269,57 @@ __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, 
       global_add(p, k[r], h, pass, 1u, v[r], v[r], v[r]);
     }
   } else {
-    // home and next bucket of every row, all eight loads in flight together
-    uint32_t b[4];
-    uint4 q[4], q2[4];
+    // First buckets of the four rows, all loads in flight together; the second
+    // is read only by lanes whose first bucket holds two keys or more and not
+    // theirs.
+    uint32_t x[4], b[4];
+    uint4 q[4];
     int slot[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      b[r] = gb_slot(gb_h(k[r]), nb);
-      const uint32_t b2 = b[r] + 1 == nb ? 0 : b[r] + 1;
-      q[r] = *reinterpret_cast<const uint4 *>(t.key + 4 * (base + b[r]));
-      q2[r] = *reinterpret_cast<const uint4 *>(t.key + 4 * (base + b2));
+      x[r] = gb_mix32(k[r]);
+      b[r] = gb_bucket1(x[r], nb);
+      q[r] = *reinterpret_cast<const uint4 *>(t.key + 4 * b[r]);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       // the all-ones key equals the empty marker: it always takes the global path
       const int hit = bucket_match(q[r], k[r]);
-      const bool home_full = bucket_match(q[r], GB_EMPTY) < 0;
-      const int hit2 = home_full ? bucket_match(q2[r], k[r]) : -1;
-      const uint32_t b2 = b[r] + 1 == nb ? 0 : b[r] + 1;
-      slot[r] = k[r] == GB_EMPTY ? -1
-              : hit >= 0         ? (int)(4 * (base + b[r])) + hit
-              : hit2 >= 0        ? (int)(4 * (base + b2)) + hit2
-                                 : -2;
+      slot[r] = !((valid >> r) & 1u) ? -3
+              : k[r] == GB_EMPTY     ? -1
+              : hit >= 0             ? (int)(4 * b[r]) + hit
+                                     : -2;
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      if (!((valid >> r) & 1u)) slot[r] = -3;
-      else if (slot[r] == -2) slot[r] = smem_find(t, base, nb, k[r], b[r]);
+      if (slot[r] == -2 && q[r].y != GB_EMPTY) {
+        b[r] = gb_bucket2(x[r], nb);
+        q[r] = *reinterpret_cast<const uint4 *>(t.key + 4 * b[r]);
+        const int hit = bucket_match(q[r], k[r]);
+        if (hit >= 0) slot[r] = (int)(4 * b[r]) + hit;
+      }
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (slot[r] == -2) slot[r] = smem_find(t.key, t.list, t.nlist, nb, k[r]);
+    // accumulator of a slot: the slot itself, or this lane's of the slot's 32
+    uint32_t acc[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      acc[r] = MODE == GB_LANE ? (uint32_t)slot[r] * 32u + (threadIdx.x & 31u) : (uint32_t)slot[r];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (slot[r] >= 0) {
-        atomicAdd(t.cnt + slot[r], 1u);
-        atomicAdd(reinterpret_cast<unsigned long long *>(t.sum) + slot[r], (unsigned long long)v[r]);
+        atomicAdd(t.cnt + acc[r], 1u);
+        smem_add64(t.slo + acc[r], t.shi + acc[r], (unsigned long long)v[r]);
       }
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (slot[r] >= 0) {
-        const longlong2 m = t.mm[slot[r]];
-        if (v[r] < m.x) atomicMin(&t.mm[slot[r]].x, v[r]);
-        if (v[r] > m.y) atomicMax(&t.mm[slot[r]].y, v[r]);
+        const longlong2 m = t.mm[acc[r]];
+        if (v[r] < m.x) atomicMin(&t.mm[acc[r]].x, v[r]);
+        if (v[r] > m.y) atomicMax(&t.mm[acc[r]].y, v[r]);
       }
     }
 #pragma unroll
@@ -257,32 +334,42 @@ __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, 
 template <int MODE>
 __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, uint32_t pass,
                                          uint64_t r0, uint64_t r1, uint64_t gw, uint64_t warps,
-                                         int lane, uint32_t base, uint32_t nb) {
+                                         int lane, uint32_t nb) {
   uint64_t done = r0;
   if (p.vec && (r0 & 3u) == 0) {
     const uint64_t q1 = r1 / 4;  // quads of rows
     const uint4 *k4 = reinterpret_cast<const uint4 *>(p.key);
     const longlong2 *v2 = reinterpret_cast<const longlong2 *>(p.val);
-    for (uint64_t b = r0 / 4 + gw * 32; b < q1; b += warps * 32) {
+    const bool split = MODE == GB_DIRECT && p.npasses > 1;
+    uint4 k = make_uint4(0, 0, 0, 0);
+    longlong2 va = make_longlong2(1, 1), vb = make_longlong2(1, 1);
+    auto load = [&](uint64_t q) {
+      if (q >= q1) return;
+      k = __ldcs(k4 + q);
+      if (p.val && !split) {
+        va = __ldcs(v2 + 2 * q);
+        vb = __ldcs(v2 + 2 * q + 1);
+      }
+    };
+    // the shared-table modes load the next step's rows while this step's are
+    // aggregated; direct updates run at 32 registers, which have no room for them
+    constexpr bool AHEAD = MODE != GB_DIRECT;
+    uint64_t b = r0 / 4 + gw * 32;
+    if (AHEAD) load(b + lane);
+    for (; b < q1; b += warps * 32) {
       const uint64_t q = b + lane;
       const bool ok = q < q1;
-      uint4 k = make_uint4(0, 0, 0, 0);
-      longlong2 va = make_longlong2(1, 1), vb = make_longlong2(1, 1);
-      if (ok) {
-        k = __ldcs(k4 + q);
-        bool need = true;
-        if (MODE == GB_DIRECT && p.npasses > 1) {
-          need = gb_pass(gb_h(k.x), p.npasses) == pass || gb_pass(gb_h(k.y), p.npasses) == pass ||
-                 gb_pass(gb_h(k.z), p.npasses) == pass || gb_pass(gb_h(k.w), p.npasses) == pass;
-        }
-        if (p.val && need) {
-          va = __ldcs(v2 + 2 * q);
-          vb = __ldcs(v2 + 2 * q + 1);
-        }
-      }
+      if (!AHEAD) load(q);
       const uint32_t kk[4] = {k.x, k.y, k.z, k.w};
+      if (split && ok && p.val &&
+          (gb_pass(gb_h(k.x), p.npasses) == pass || gb_pass(gb_h(k.y), p.npasses) == pass ||
+           gb_pass(gb_h(k.z), p.npasses) == pass || gb_pass(gb_h(k.w), p.npasses) == pass)) {
+        va = __ldcs(v2 + 2 * q);
+        vb = __ldcs(v2 + 2 * q + 1);
+      }
       const long long vv[4] = {va.x, va.y, vb.x, vb.y};
-      gb_rows4<MODE>(p, t, pass, kk, vv, ok ? 0xFu : 0u, base, nb);
+      if (AHEAD) load(q + warps * 32);
+      gb_rows4<MODE>(p, t, pass, kk, vv, ok ? 0xFu : 0u, nb);
     }
     done = q1 * 4;
   }
@@ -299,7 +386,7 @@ __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, 
       kk[r] = in ? p.key[i] : 0u;
       vv[r] = (in && p.val) ? (long long)p.val[i] : 1ll;
     }
-    gb_rows4<MODE>(p, t, pass, kk, vv, valid, base, nb);
+    gb_rows4<MODE>(p, t, pass, kk, vv, valid, nb);
   }
 }
 
@@ -307,54 +394,99 @@ __device__ __forceinline__ SmemTable gb_smem_table(unsigned char *smem) {
   SmemTable t;
   t.key = reinterpret_cast<uint32_t *>(smem);
   t.cnt = t.key + GB_SMEM_SLOTS;
-  t.sum = reinterpret_cast<long long *>(t.cnt + GB_SMEM_SLOTS);
-  t.mm = reinterpret_cast<longlong2 *>(t.sum + GB_SMEM_SLOTS);
+  t.slo = t.cnt + GB_SMEM_SLOTS;
+  t.shi = t.slo + GB_SMEM_SLOTS;
+  t.mm = reinterpret_cast<longlong2 *>(t.shi + GB_SMEM_SLOTS);
   t.list = nullptr;
   t.nlist = nullptr;
   return t;
 }
 
-__device__ __forceinline__ void gb_clear_slot(const SmemTable &t, uint32_t i) {
-  t.key[i] = GB_EMPTY;
+__device__ __forceinline__ void gb_clear_acc(const SmemTable &t, uint32_t i) {
   t.cnt[i] = 0;
-  t.sum[i] = 0;
+  t.slo[i] = 0;
+  t.shi[i] = 0;
   t.mm[i] = make_longlong2(INT64_MAX, INT64_MIN);
 }
 
-// Shared buckets of this lane: its warp's replica (GB_WARP) or the CTA table.
-__device__ __forceinline__ void gb_buckets(int mode, uint32_t wrep, uint32_t *base, uint32_t *nb) {
-  *base = 0;
-  *nb = GB_SMEM_SLOTS / 4;
-  if (mode == GB_WARP) {
-    const int lane = threadIdx.x & 31;
-    *nb = GB_WARP_SLOTS / 4 / wrep;
-    *base = (threadIdx.x >> 5) * (GB_WARP_SLOTS / 4) + (lane / (32 / wrep)) * *nb;
+__device__ __forceinline__ void gb_clear_all(const SmemTable &t) {
+  for (uint32_t i = threadIdx.x; i < GB_SMEM_SLOTS; i += GB_THREADS) {
+    t.key[i] = GB_EMPTY;
+    gb_clear_acc(t, i);
   }
 }
 
-// Persistent CTAs over all rows.  In GB_WARP mode each warp's 192 slots form
-// p.wrep private replicas, one per group of 32 / p.wrep lanes.
+__device__ __forceinline__ unsigned long long gb_sum(const SmemTable &t, uint32_t i) {
+  return (unsigned long long)t.shi[i] << 32 | t.slo[i];
+}
+
+// Buckets of the shared table in a mode.
+__device__ __forceinline__ uint32_t gb_nbuckets(int mode) {
+  return (mode == GB_LANE ? GB_LANE_SLOTS : GB_SMEM_SLOTS) / 4;
+}
+
+// Merges the claimed slots into the global table: nl slots of t.list, or
+// every occupied slot of the table when list is false; reset clears them for
+// the next rows.  A GB_LANE slot's 32 accumulators are reduced by one warp.
+__device__ __forceinline__ void gb_flush(const GbParams &p, const SmemTable &t, int mode, bool list,
+                                         uint32_t nl, bool reset) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t n = list ? nl : (mode == GB_LANE ? GB_LANE_SLOTS : GB_SMEM_SLOTS);
+  if (mode == GB_LANE) {
+    for (uint32_t i = threadIdx.x >> 5; i < n; i += GB_WARPS) {
+      const uint32_t j = list ? t.list[i] : i;
+      const uint32_t k = t.key[j];
+      if (k == GB_EMPTY) continue;
+      const uint32_t a = 32 * j + lane;
+      uint32_t cnt = t.cnt[a];
+      unsigned long long sum = gb_sum(t, a);
+      long long mn = t.mm[a].x, mx = t.mm[a].y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      }
+      if (lane == 0) global_add(p, k, gb_h(k), 0, cnt, (long long)sum, mn, mx);
+      if (reset) {
+        gb_clear_acc(t, a);
+        if (lane == 0) t.key[j] = GB_EMPTY;
+      }
+    }
+    return;
+  }
+  // the CTAs of one launch hold the same groups in about the same slots: each
+  // starts elsewhere in its table, so that they do not all update one group
+  const uint32_t first = list ? 0u : (uint32_t)((uint64_t)n * blockIdx.x / gridDim.x);
+  for (uint32_t i = threadIdx.x; i < n; i += GB_THREADS) {
+    const uint32_t j = list ? t.list[i] : (i + first < n ? i + first : i + first - n);
+    const uint32_t k = t.key[j];
+    if (k == GB_EMPTY) continue;
+    global_add(p, k, gb_h(k), 0, t.cnt[j], (long long)gb_sum(t, j), t.mm[j].x, t.mm[j].y);
+    if (reset) {
+      t.key[j] = GB_EMPTY;
+      gb_clear_acc(t, j);
+    }
+  }
+}
+
+// Persistent CTAs over all rows.
 template <int MODE>
 __global__ void __launch_bounds__(GB_THREADS, MODE == GB_DIRECT ? 2 : 1)
 k_gb_aggregate(GbParams p, uint32_t pass) {
   extern __shared__ __align__(16) unsigned char gb_smem[];
   const SmemTable t = gb_smem_table(gb_smem);
   if (MODE != GB_DIRECT) {
-    for (uint32_t i = threadIdx.x; i < GB_SMEM_SLOTS; i += GB_THREADS) gb_clear_slot(t, i);
+    gb_clear_all(t);
     __syncthreads();
   }
-  uint32_t base, nb;
-  gb_buckets(MODE, p.wrep, &base, &nb);
   const uint64_t warps = (uint64_t)gridDim.x * GB_WARPS;
   const uint64_t gw = (uint64_t)blockIdx.x * GB_WARPS + (threadIdx.x >> 5);
-  gb_range<MODE>(p, t, pass, 0, p.n, gw, warps, threadIdx.x & 31, base, nb);
+  gb_range<MODE>(p, t, pass, 0, p.n, gw, warps, threadIdx.x & 31, gb_nbuckets(MODE));
   if (MODE != GB_DIRECT) {
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < GB_SMEM_SLOTS; i += GB_THREADS) {
-      const uint32_t k = t.key[i];
-      if (k != GB_EMPTY)
-        global_add(p, k, gb_h(k), 0, t.cnt[i], t.sum[i], t.mm[i].x, t.mm[i].y);
-    }
+    gb_flush(p, t, MODE, false, 0, false);
   }
 }
 
@@ -368,7 +500,7 @@ __global__ void __launch_bounds__(GB_THREADS, 1) k_gb_chunks(GbParams p, uint64_
   SmemTable t = gb_smem_table(gb_smem);
   t.list = reinterpret_cast<uint16_t *>(gb_smem + GB_SMEM_BYTES);
   t.nlist = &s_nlist;
-  for (uint32_t i = threadIdx.x; i < GB_SMEM_SLOTS; i += GB_THREADS) gb_clear_slot(t, i);
+  gb_clear_all(t);
   if (threadIdx.x == 0) s_nlist = 0;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = threadIdx.x >> 5;
@@ -387,15 +519,9 @@ __global__ void __launch_bounds__(GB_THREADS, 1) k_gb_chunks(GbParams p, uint64_
     const uint64_t it = s_item;
     if (it >= nchunks) break;
     const uint64_t r0 = it * chunk, r1 = min(r0 + chunk, p.n);
-    gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_WARPS, lane, 0, GB_SMEM_SLOTS / 4);
+    gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_WARPS, lane, gb_nbuckets(GB_SMEM));
     __syncthreads();
-    const uint32_t nl = s_nlist;
-    for (uint32_t i = threadIdx.x; i < nl; i += GB_THREADS) {
-      const uint32_t j = t.list[i];
-      const uint32_t k = t.key[j];
-      global_add(p, k, gb_h(k), 0, t.cnt[j], t.sum[j], t.mm[j].x, t.mm[j].y);
-      gb_clear_slot(t, j);
-    }
+    gb_flush(p, t, GB_SMEM, true, s_nlist, true);
     __syncthreads();
     if (threadIdx.x == 0) s_nlist = 0;
   }
@@ -427,7 +553,6 @@ __device__ __forceinline__ GbParams gbb_params(const pd_gb_batch &b, const pd_gb
   p.gtab = b.gtab + 4 * in.slot0;
   p.sub_cap = in.slots;
   p.npasses = 1;
-  p.wrep = in.wrep;
   p.d_error = b.d_error;
   return p;
 }
@@ -452,7 +577,7 @@ __global__ void __launch_bounds__(GB_THREADS, 1) k_gbb_aggregate(pd_gb_batch b) 
   SmemTable t = gb_smem_table(gb_smem);
   t.list = reinterpret_cast<uint16_t *>(gb_smem + GB_SMEM_BYTES);
   t.nlist = &s_nlist;
-  for (uint32_t i = threadIdx.x; i < GB_SMEM_SLOTS; i += GB_THREADS) gb_clear_slot(t, i);
+  gb_clear_all(t);
   if (threadIdx.x == 0) s_nlist = 0;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = threadIdx.x >> 5;
@@ -474,20 +599,13 @@ __global__ void __launch_bounds__(GB_THREADS, 1) k_gbb_aggregate(pd_gb_batch b) 
     const GbParams p = gbb_params(b, in);
     const uint64_t r0 = item.y, r1 = min((uint64_t)item.y + b.rows_per_item, in.n);
     const int mode = (int)in.mode;
-    uint32_t base, nb;
-    gb_buckets(mode, in.wrep, &base, &nb);
-    if (mode == GB_WARP) gb_range<GB_WARP>(p, t, 0, r0, r1, warp, GB_WARPS, lane, base, nb);
-    else if (mode == GB_SMEM) gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_WARPS, lane, base, nb);
-    else gb_range<GB_DIRECT>(p, t, 0, r0, r1, warp, GB_WARPS, lane, base, nb);
+    const uint32_t nb = gb_nbuckets(mode);
+    if (mode == GB_LANE) gb_range<GB_LANE>(p, t, 0, r0, r1, warp, GB_WARPS, lane, nb);
+    else if (mode == GB_SMEM) gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_WARPS, lane, nb);
+    else gb_range<GB_DIRECT>(p, t, 0, r0, r1, warp, GB_WARPS, lane, nb);
     if (mode != GB_DIRECT) {
       __syncthreads();
-      const uint32_t nl = s_nlist;
-      for (uint32_t i = threadIdx.x; i < nl; i += GB_THREADS) {
-        const uint32_t j = t.list[i];
-        const uint32_t k = t.key[j];
-        global_add(p, k, gb_h(k), 0, t.cnt[j], t.sum[j], t.mm[j].x, t.mm[j].y);
-        gb_clear_slot(t, j);
-      }
+      gb_flush(p, t, mode, true, s_nlist, true);
       __syncthreads();
       if (threadIdx.x == 0) s_nlist = 0;
     }
@@ -984,7 +1102,7 @@ __global__ void k_vrange_pick(const long long *mm, uint64_t n, uint64_t *n_pay, 
 
 struct GbLayout {
   int mode;
-  uint32_t sub_cap, npasses, wrep;
+  uint32_t sub_cap, npasses;
   uint32_t part_bits;   // GB_PART: hash partitions 2^part_bits
   size_t gtab, ngroups, ckey, cslot, skey, sslot, sort_ws, pkey, pval, vrange, total;
 };
@@ -1036,7 +1154,7 @@ bool gb_layout(const pimdal_aggr_arguments_t *a, GbLayout *l, const GbTune *tune
     sa.nr_elements = a->size;
     if (pimdal_sort_workspace_size(&sa, &w)) return false;
     l->mode = -1;
-    l->sub_cap = l->npasses = l->wrep = 0;
+    l->sub_cap = l->npasses = 0;
     l->vrange = o; o += 256;  // min, max, rows of the payload and row-id paths
     l->ngroups = o; o += pd_align_up(8 * (pd_ceil_div(a->size, SR_TILE) + 1), 256);
     l->skey = o; o += pd_align_up(4 * a->size, 256);
@@ -1047,7 +1165,7 @@ bool gb_layout(const pimdal_aggr_arguments_t *a, GbLayout *l, const GbTune *tune
   }
   uint64_t expect = a->expected_groups ? a->expected_groups : std::min<uint64_t>(a->size, 1ull << 22);
   expect = std::max<uint64_t>(expect, 1);
-  l->mode = expect <= GB_WARP_MAX_GROUPS ? GB_WARP : expect <= GB_SMEM_MAX_GROUPS ? GB_SMEM
+  l->mode = expect <= GB_LANE_MAX_GROUPS ? GB_LANE : expect <= GB_SMEM_MAX_GROUPS ? GB_SMEM
           : gb_force_direct() ? GB_DIRECT : GB_PART;
   if (tune && tune->mode >= 0 && l->mode >= GB_DIRECT) l->mode = tune->mode;
   l->part_bits = 0;
@@ -1059,8 +1177,6 @@ bool gb_layout(const pimdal_aggr_arguments_t *a, GbLayout *l, const GbTune *tune
       b = tune->part_bits;
     l->part_bits = b;
   }
-  // GB_WARP replicas: keep each replica's load at or below 1/3
-  l->wrep = expect <= 16 ? 4 : expect <= 32 ? 2 : 1;
   // load factor 1/2 for the small tables, 3/4 for the large ones
   uint64_t slots = l->mode >= GB_DIRECT ? expect + expect / 3 + 1 : 2 * expect;
   slots = std::max<uint64_t>(slots, 2048);
@@ -1094,10 +1210,8 @@ bool gb_layout(const pimdal_aggr_arguments_t *a, GbLayout *l, const GbTune *tune
 
 }  // namespace
 
-void pd_gb_mode(uint64_t expect, uint32_t *mode, uint32_t *wrep) {
-  expect = std::max<uint64_t>(expect, 1);
-  *mode = expect <= GB_WARP_MAX_GROUPS ? GB_WARP : expect <= GB_SMEM_MAX_GROUPS ? GB_SMEM : GB_DIRECT;
-  *wrep = expect <= 16 ? 4 : expect <= 32 ? 2 : 1;
+uint32_t pd_gb_mode(uint64_t expect) {
+  return expect <= GB_LANE_MAX_GROUPS ? GB_LANE : expect <= GB_SMEM_MAX_GROUPS ? GB_SMEM : GB_DIRECT;
 }
 
 size_t pd_gb_batch_shared_bytes() { return GB_SMEM_BYTES + 2 * GB_SMEM_SLOTS; }
@@ -1368,7 +1482,6 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
   p.gtab = (unsigned long long *)(ws + l.gtab);
   p.sub_cap = l.sub_cap;
   p.npasses = l.npasses;
-  p.wrep = l.wrep;
   p.ngroups = (unsigned long long *)(ws + l.ngroups);
   p.ckey = (uint32_t *)(ws + l.ckey);
   p.cslot = (uint32_t *)(ws + l.cslot);
@@ -1412,7 +1525,7 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
   } else {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_GROUP, s);
     const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count);
-    auto k = l.mode == GB_WARP ? k_gb_aggregate<GB_WARP> : k_gb_aggregate<GB_SMEM>;
+    auto k = l.mode == GB_LANE ? k_gb_aggregate<GB_LANE> : k_gb_aggregate<GB_SMEM>;
     PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GB_SMEM_BYTES));
     k<<<grid ? grid : 1, GB_THREADS, GB_SMEM_BYTES, s>>>(p, 0);
   }

@@ -117,6 +117,37 @@ float pd_time_call(pimdal_ctx *ctx, cudaStream_t s, F run) {
   return st == PIMDAL_OK ? ms : -1.f;
 }
 
+// Launches a kernel that begins with pd_grid_dep().  Such a kernel may be
+// brought onto the SMs while the one before it in the stream is still running,
+// which hides its launch (about 2 us of a dependent launch): its threads wait
+// in pd_grid_dep() until everything before it is complete and visible.  After
+// anything but a kernel (a copy, a memset, an event) the launch is an
+// ordinary one, as it is with early = false.  cluster > 1 makes clusters of
+// that many CTAs.
+template <typename... P, typename... A>
+cudaError_t pd_launch_early(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                            cudaStream_t s, unsigned cluster, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = early;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t pd_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                      unsigned cluster, A... args) {
+  return pd_launch_early(true, kernel, grid, block, smem, s, cluster, args...);
+}
+
 // Next lookback epoch (1..65535); clears the status words when it wraps.
 uint32_t pd_next_epoch(pimdal_ctx *ctx, cudaStream_t stream, int *status);
 
@@ -135,6 +166,17 @@ PD_HD uint64_t pd_ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 // ---------------------------------------------------------------------------
 // Device helpers
 // ---------------------------------------------------------------------------
+// First statement of a kernel launched by pd_launch: lets the next kernel of the
+// stream come onto the SMs, then waits for all that was launched before.
+// Nothing in global memory may be read or written before the wait.
+__device__ __forceinline__ void pd_grid_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pd_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pd_grid_dep() {
+  pd_grid_trigger();
+  pd_grid_wait();
+}
 __device__ __forceinline__ void pd_store_release_u64(uint64_t *p, uint64_t v) {
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }

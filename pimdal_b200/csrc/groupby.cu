@@ -99,6 +99,7 @@ __device__ __forceinline__ uint32_t gb_slot(uint64_t h, uint32_t cap) {
 }
 
 __global__ void __launch_bounds__(256) k_gb_init(GbParams p) {
+  pd_grid_dep();
   const uint64_t slots = (uint64_t)p.sub_cap * p.npasses;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   ulonglong2 *t = reinterpret_cast<ulonglong2 *>(p.gtab);
@@ -475,12 +476,14 @@ __device__ __forceinline__ void gb_flush(const GbParams &p, const SmemTable &t, 
 template <int MODE>
 __global__ void __launch_bounds__(GB_THREADS, MODE == GB_DIRECT ? 2 : 1)
 k_gb_aggregate(GbParams p, uint32_t pass) {
+  pd_grid_trigger();
   extern __shared__ __align__(16) unsigned char gb_smem[];
   const SmemTable t = gb_smem_table(gb_smem);
   if (MODE != GB_DIRECT) {
     gb_clear_all(t);
     __syncthreads();
   }
+  pd_grid_wait();
   const uint64_t warps = (uint64_t)gridDim.x * GB_WARPS;
   const uint64_t gw = (uint64_t)blockIdx.x * GB_WARPS + (threadIdx.x >> 5);
   gb_range<MODE>(p, t, pass, 0, p.n, gw, warps, threadIdx.x & 31, gb_nbuckets(MODE));
@@ -495,6 +498,7 @@ k_gb_aggregate(GbParams p, uint32_t pass) {
 // slots it claimed are flushed to the global table and reset.
 __global__ void __launch_bounds__(GB_THREADS, 1) k_gb_chunks(GbParams p, uint64_t chunk,
                                                              uint32_t *claim) {
+  pd_grid_dep();
   extern __shared__ __align__(16) unsigned char gb_smem[];
   __shared__ uint32_t s_item, s_nlist;
   SmemTable t = gb_smem_table(gb_smem);
@@ -700,6 +704,7 @@ __global__ void __launch_bounds__(256) k_gbb_gather(pd_gb_batch b) {
 
 // Occupied slots -> (key, slot) list (order is restored by the sort that follows).
 __global__ void __launch_bounds__(256) k_gb_compact(GbParams p) {
+  pd_grid_dep();
   const uint64_t slots = (uint64_t)p.sub_cap * p.npasses;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
@@ -730,6 +735,7 @@ struct GatherParams {
 };
 
 __global__ void __launch_bounds__(256) k_gb_gather(GatherParams g) {
+  pd_grid_dep();
   const uint64_t n = *g.ngroups;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *g.d_count = n;
@@ -797,6 +803,7 @@ __device__ __forceinline__ bool sr_active(SegParams &p) {
 }
 
 __global__ void __launch_bounds__(SR_THREADS) k_sr_heads(SegParams p) {
+  pd_grid_dep();
   __shared__ uint32_t s_red[SR_THREADS / 32];
   if (!sr_active(p)) return;
   for (uint64_t tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
@@ -818,6 +825,7 @@ __global__ void __launch_bounds__(SR_THREADS) k_sr_heads(SegParams p) {
 }
 
 __global__ void __launch_bounds__(1024) k_sr_scan(SegParams p) {
+  pd_grid_dep();
   __shared__ uint64_t s_w[32];
   __shared__ uint64_t s_carry;
   if (!sr_active(p)) return;
@@ -852,6 +860,7 @@ __global__ void __launch_bounds__(1024) k_sr_scan(SegParams p) {
 }
 
 __global__ void __launch_bounds__(256) k_sr_init(SegParams p) {
+  pd_grid_dep();
   if (!sr_active(p)) return;
   const uint64_t lim = min(*p.d_count, p.cap);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -925,6 +934,7 @@ __device__ __forceinline__ void sr_store(const SegParams &p, uint64_t g, uint32_
 // 3 CTAs per SM (80 registers, a 28-byte spill) instead of 2 at 126:
 // 1.26 -> 1.10 ms over 2^28 sorted rows (4 CTAs at 64 spilled more, 1.22).
 __global__ void __launch_bounds__(SR_THREADS, 3) k_gb_segreduce(SegParams p) {
+  pd_grid_dep();
   __shared__ uint32_t s_heads[SR_THREADS / 32];
   __shared__ SrSeg s_seg[SR_THREADS / 32];
   if (!sr_active(p)) return;
@@ -1043,11 +1053,13 @@ __global__ void __launch_bounds__(SR_THREADS, 3) k_gb_segreduce(SegParams p) {
 
 // Minimum and maximum of the values (mm[0], mm[1]).
 __global__ void k_vrange_init(long long *mm) {
+  pd_grid_dep();
   mm[0] = INT64_MAX;
   mm[1] = INT64_MIN;
 }
 
 __global__ void __launch_bounds__(256) k_vrange(const long long *v, uint64_t n, long long *mm) {
+  pd_grid_dep();
   long long lo = INT64_MAX, hi = INT64_MIN;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1095,6 +1107,7 @@ __global__ void __launch_bounds__(256) k_vrange(const long long *v, uint64_t n, 
 // The payload path takes the rows when max - min fits 32 bits, else the
 // row-id path does.
 __global__ void k_vrange_pick(const long long *mm, uint64_t n, uint64_t *n_pay, uint64_t *n_idx) {
+  pd_grid_dep();
   const bool fits = (unsigned long long)mm[1] - (unsigned long long)mm[0] <= 0xFFFFFFFFull;
   *n_pay = fits ? n : 0;
   *n_idx = fits ? 0 : n;
@@ -1423,19 +1436,19 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
       const unsigned sr_grid = (unsigned)std::min<uint64_t>(q.tiles, ctx->sm_count * 8ull);
       {
         pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-        k_sr_heads<<<sr_grid, SR_THREADS, 0, s>>>(q);
+        PD_CHECK_CUDA(pd_launch(k_sr_heads, sr_grid, SR_THREADS, 0, s, 1, q));
       }
       {
         pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-        k_sr_scan<<<1, 1024, 0, s>>>(q);
+        PD_CHECK_CUDA(pd_launch(k_sr_scan, 1, 1024, 0, s, 1, q));
       }
       {
         pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-        k_sr_init<<<ctx->sm_count * 8, 256, 0, s>>>(q);
+        PD_CHECK_CUDA(pd_launch(k_sr_init, ctx->sm_count * 8, 256, 0, s, 1, q));
       }
       {
         pd_launch_scope sc(ctx, PIMDAL_KERNEL_SEGREDUCE, s);
-        k_gb_segreduce<<<sr_grid, SR_THREADS, 0, s>>>(q);
+        PD_CHECK_CUDA(pd_launch(k_gb_segreduce, sr_grid, SR_THREADS, 0, s, 1, q));
       }
       return pd_launch_status(ctx);
     };
@@ -1446,16 +1459,16 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
     }
     {
       pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-      k_vrange_init<<<1, 1, 0, s>>>(mm);
+      PD_CHECK_CUDA(pd_launch(k_vrange_init, 1, 1, 0, s, 1, mm));
     }
     {
       pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
       const unsigned g = (unsigned)std::min<uint64_t>(pd_ceil_div(a->size, 512), ctx->sm_count * 8ull);
-      k_vrange<<<g, 256, 0, s>>>((const long long *)a->in_val, a->size, mm);
+      PD_CHECK_CUDA(pd_launch(k_vrange, g, 256, 0, s, 1, (const long long *)a->in_val, a->size, mm));
     }
     {
       pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-      k_vrange_pick<<<1, 1, 0, s>>>(mm, a->size, n_pay, n_idx);
+      PD_CHECK_CUDA(pd_launch(k_vrange_pick, 1, 1, 0, s, 1, mm, a->size, n_pay, n_idx));
     }
     sa.out_ptr = (uint32_t *)(ws + l.sslot);
     p.sidx = (const uint32_t *)(ws + l.sslot);
@@ -1490,7 +1503,7 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
   const unsigned init_grid = (unsigned)std::min<uint64_t>(pd_ceil_div(cap, 256), ctx->sm_count * 8ull);
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_gb_init<<<init_grid, 256, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_gb_init, init_grid, 256, 0, s, 1, p));
   }
   const uint64_t want = pd_ceil_div(a->size, (uint64_t)GB_THREADS * 4);
   if (l.mode == GB_PART) {
@@ -1515,23 +1528,23 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
     const size_t smem = pd_gb_batch_shared_bytes();
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_GROUP, s);
     PD_CHECK_CUDA(cudaFuncSetAttribute(k_gb_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_gb_chunks<<<grid ? grid : 1, GB_THREADS, smem, s>>>(p, chunk, ctx->d_counters + PD_COUNTER_GROUP);
+    PD_CHECK_CUDA(pd_launch(k_gb_chunks, grid ? grid : 1, GB_THREADS, smem, s, 1, p, chunk, ctx->d_counters + PD_COUNTER_GROUP));
   } else if (l.mode == GB_DIRECT) {
     const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count * 2);
     for (uint32_t q = 0; q < l.npasses; ++q) {
       pd_launch_scope sc(ctx, PIMDAL_KERNEL_GROUP, s);
-      k_gb_aggregate<GB_DIRECT><<<grid ? grid : 1, GB_THREADS, 0, s>>>(p, q);
+      PD_CHECK_CUDA(pd_launch(k_gb_aggregate<GB_DIRECT>, grid ? grid : 1, GB_THREADS, 0, s, 1, p, q));
     }
   } else {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_GROUP, s);
     const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count);
     auto k = l.mode == GB_LANE ? k_gb_aggregate<GB_LANE> : k_gb_aggregate<GB_SMEM>;
     PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GB_SMEM_BYTES));
-    k<<<grid ? grid : 1, GB_THREADS, GB_SMEM_BYTES, s>>>(p, 0);
+    PD_CHECK_CUDA(pd_launch(k, grid ? grid : 1, GB_THREADS, GB_SMEM_BYTES, s, 1, p, 0u));
   }
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_gb_compact<<<init_grid, 256, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_gb_compact, init_grid, 256, 0, s, 1, p));
   }
   sa.nr_elements = cap;  // upper bound; the real count is read on the device
   sa.in = p.ckey;
@@ -1556,7 +1569,7 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
   g.d_error = ctx->d_error;
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_gb_gather<<<init_grid, 256, 0, s>>>(g);
+    PD_CHECK_CUDA(pd_launch(k_gb_gather, init_grid, 256, 0, s, 1, g));
   }
   return pd_launch_status(ctx);
 }

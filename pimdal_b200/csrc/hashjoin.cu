@@ -92,16 +92,12 @@ struct JoinParams {
   uint32_t bits, part_bits;
   uint32_t *side_count;
   uint32_t *dup_flag;           // set by the build when a key occurs twice
-  // build side (partition p = rows [boff[p], boff[p+1]))
+  // build side
   const uint32_t *bkey, *bpay;  // bpay NULL: payload = row id
-  const uint32_t *boff;         // device partition offsets (NULL: whole input)
   uint64_t nb;
   // probe side
   const uint32_t *pkey, *prow;  // prow NULL: row id = index
-  const uint32_t *poff;
-  const uint32_t *tilebase;     // first global tile of each partition
   uint64_t np;
-  uint32_t part;
   // output
   uint32_t *out_pay, *out_row;
   uint64_t cap;
@@ -110,22 +106,11 @@ struct JoinParams {
   uint32_t *claim;
   uint32_t *d_error;
   uint64_t *d_count;
-  uint64_t total_tiles;         // for d_count (direct path)
 };
-
-__device__ __forceinline__ void part_range(const uint32_t *off, uint32_t p, uint64_t n,
-                                           uint64_t *lo, uint64_t *hi) {
-  if (off) {
-    *lo = off[p];
-    *hi = off[p + 1];
-  } else {
-    *lo = 0;
-    *hi = n;
-  }
-}
 
 // Fills the table region with the empty word and zeroes the side count.
 __global__ void __launch_bounds__(256) k_hj_clear(JoinParams p) {
+  pd_grid_dep();
   const uint64_t n = 1ull << p.bits;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   ulonglong2 e = make_ulonglong2(HJ_EMPTY, HJ_EMPTY);
@@ -178,10 +163,9 @@ __device__ __forceinline__ void hj_insert(const JoinParams &p, uint32_t k, uint3
 }
 
 __global__ void __launch_bounds__(256) k_hj_build(JoinParams p) {
-  uint64_t lo, hi;
-  part_range(p.boff, p.part, p.nb, &lo, &hi);
+  pd_grid_dep();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += stride)
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.nb; i += stride)
     hj_insert(p, p.bkey[i], p.bpay ? p.bpay[i] : (uint32_t)i);
 }
 
@@ -425,12 +409,10 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
 }
 
 __global__ void __launch_bounds__(HJ_THREADS, PD_HJ_MIN_CTAS) k_hj_probe(JoinParams p) {
+  pd_grid_dep();
   __shared__ uint64_t s_tile;
   const int tid = threadIdx.x;
-  uint64_t lo, hi;
-  part_range(p.poff, p.part, p.np, &lo, &hi);
-  const uint64_t tiles = pd_ceil_div(hi - lo, HJ_TILE);
-  const uint64_t gbase = p.tilebase ? p.tilebase[p.part] : 0;
+  const uint64_t tiles = pd_ceil_div(p.np, HJ_TILE);
   const uint32_t side = *p.side_count;
   const bool stop_first = *p.dup_flag == 0;
   while (true) {
@@ -445,39 +427,12 @@ __global__ void __launch_bounds__(HJ_THREADS, PD_HJ_MIN_CTAS) k_hj_probe(JoinPar
     __syncthreads();
     const uint64_t tl = s_tile;
     if (tl >= tiles) break;
-    hj_probe_tile(p, lo + tl * HJ_TILE, hi, gbase + tl, side, stop_first, false);
+    hj_probe_tile(p, tl * HJ_TILE, p.np, tl, side, stop_first, false);
+    // the inclusive count this thread has just published (inside the tile's
+    // code the count costs registers that it does not have: 1% slower)
+    if (tl == tiles - 1 && tid == 0)
+      *p.d_count = pd_load_relaxed_u64(p.status + tl) & PD_STATUS_VALUE_MASK;
   }
-}
-
-// Total match count: the inclusive prefix of the last global probe tile.
-__global__ void k_hj_count(const uint64_t *status, const uint32_t *tilebase, uint32_t parts,
-                           uint64_t total_tiles, uint32_t epoch, uint64_t *d_count) {
-  uint64_t tiles = tilebase ? tilebase[parts] : total_tiles;
-  uint64_t v = 0;
-  if (tiles) {
-    uint64_t w = pd_load_relaxed_u64(status + tiles - 1);
-    v = w & PD_STATUS_VALUE_MASK;
-  }
-  *d_count = v;
-}
-
-// Exclusive offsets (uint32, P+1 entries) of two partitioned relations and the
-// first global probe tile of each partition.
-__global__ void k_hj_offsets(const uint32_t *boffs, const uint32_t *poffs, uint32_t parts,
-                             uint64_t nb, uint64_t np, uint32_t *boff, uint32_t *poff,
-                             uint32_t *tilebase) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  uint64_t t = 0;
-  for (uint32_t q = 0; q < parts; ++q) {
-    boff[q] = boffs[q];
-    poff[q] = poffs[q];
-    tilebase[q] = (uint32_t)t;
-    uint64_t end = (q + 1 < parts) ? poffs[q + 1] : np;
-    t += pd_ceil_div(end - poffs[q], HJ_TILE);
-  }
-  boff[parts] = (uint32_t)nb;
-  poff[parts] = (uint32_t)np;
-  tilebase[parts] = (uint32_t)t;
 }
 
 // ---------------------------------------------------------------------------
@@ -873,14 +828,11 @@ __global__ void __launch_bounds__(HJS_THREADS, 1) k_hjs_join(JoinSmemParams p) {
   if (overflow) atomicOr(p.d_error, PD_DEVERR_CAPACITY);
 }
 
-#ifndef PD_HJ_ONE_TABLE
-#define PD_HJ_ONE_TABLE 1
-#endif
 
 struct HjLayout {
   uint32_t bits, part_bits;
   bool smem;  // shared-memory partitions (k_hjs_join)
-  size_t table, side, boff, poff, tilebase, bk, bp, pk, pr, sort_ws, total;
+  size_t table, side, boff, poff, bk, bp, pk, pr, sort_ws, total;
 };
 
 // Shared-memory partitions: partitioned copies of both relations, their
@@ -892,7 +844,7 @@ bool hjs_layout(const pimdal_hash_join_arguments_t *a, HjLayout *l) {
   l->bits = 0;
   const size_t offs = pd_align_up(4 * ((1ull << pb) + 1), 256);
   size_t o = 0;
-  l->table = l->side = l->tilebase = 0;
+  l->table = l->side = 0;
   l->boff = o; o += offs;
   l->poff = o; o += offs;
   l->bk = o; o += pd_align_up(4 * a->size_build, 256);
@@ -927,17 +879,11 @@ bool hj_layout(const pimdal_hash_join_arguments_t *a, HjLayout *l) {
   }
   if (pb > 8 || pb >= bits) return false;
   l->part_bits = pb;
-#if PD_HJ_ONE_TABLE
   l->bits = bits;  // one table; partition q's rows touch only its slice q
-#else
-  l->bits = bits - pb;  // slots of one partition's table
-#endif
   size_t o = 0;
   l->table = o; o += pd_align_up(8ull << l->bits, 256);
   l->side = o; o += 256;
-  l->boff = o; o += pd_align_up(4 * 257, 256);
-  l->poff = o; o += pd_align_up(4 * 257, 256);
-  l->tilebase = o; o += pd_align_up(4 * 257, 256);
+  l->boff = l->poff = 0;
   l->bk = l->bp = l->pk = l->pr = l->sort_ws = 0;
   if (pb) {
     l->bk = o; o += pd_align_up(4 * a->size_build, 256);
@@ -1132,14 +1078,11 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
   char *ws = (char *)pd_workspace(ctx, l.total, s, &st);
   if (!ws) return st;
   if (l.smem) return hjs_run(ctx, a, l, ws, d_result, s);
-  const uint32_t parts = 1u << l.part_bits;
-  const uint64_t total_tiles_direct = pd_ceil_div(a->size_probe, HJ_TILE);
-  if (total_tiles_direct + parts > PD_STATUS_WORDS) return PIMDAL_ERR_ARG;
+  if (pd_ceil_div(a->size_probe, HJ_TILE) > PD_STATUS_WORDS) return PIMDAL_ERR_ARG;
 
   JoinParams p{};
   p.table = (unsigned long long *)(ws + l.table);
   p.bits = l.bits;
-  p.part_bits = l.part_bits;
   p.side_count = (uint32_t *)(ws + l.side);
   p.dup_flag = (uint32_t *)(ws + l.side) + 2;
   p.nb = a->size_build;
@@ -1161,34 +1104,22 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
     sa.layout = PIMDAL_LAYOUT_COLUMNS;
     sa.begin_bit = 32 - l.part_bits;
     sa.end_bit = 32;
-    uint32_t *boffs, *poffs;
     sa.nr_elements = a->size_build;
     sa.in = a->build_key;
     sa.in_ptr = a->build_payload;
     sa.out = ws + l.bk;
     sa.out_ptr = (uint32_t *)(ws + l.bp);
-    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s, &boffs))) return st;
-    // the build offsets live in the sort workspace: save them before reuse
-    uint32_t *boff = (uint32_t *)(ws + l.boff), *poff = (uint32_t *)(ws + l.poff);
-    PD_CHECK_CUDA(cudaMemcpyAsync(boff, boffs, 4 * parts, cudaMemcpyDeviceToDevice, s));
+    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s, nullptr))) return st;
     sa.nr_elements = a->size_probe;
     sa.in = a->probe_key;
     sa.in_ptr = a->probe_ptr;
     sa.out = ws + l.pk;
     sa.out_ptr = (uint32_t *)(ws + l.pr);
-    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s, &poffs))) return st;
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-      k_hj_offsets<<<1, 32, 0, s>>>(boff, poffs, parts, a->size_build, a->size_probe, boff, poff,
-                                    (uint32_t *)(ws + l.tilebase));
-    }
+    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s, nullptr))) return st;
     p.bkey = (const uint32_t *)(ws + l.bk);
     p.bpay = (const uint32_t *)(ws + l.bp);
     p.pkey = (const uint32_t *)(ws + l.pk);
     p.prow = (const uint32_t *)(ws + l.pr);
-    p.boff = boff;
-    p.poff = poff;
-    p.tilebase = (const uint32_t *)(ws + l.tilebase);
   } else {
     p.bkey = (const uint32_t *)a->build_key;
     p.bpay = a->build_payload;
@@ -1198,54 +1129,26 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
   const unsigned clear_grid = (unsigned)std::min<uint64_t>(pd_ceil_div(1ull << l.bits, 512), ctx->sm_count * 8ull);
   const unsigned build_grid = ctx->sm_count * 8;
   const int pgrid = probe_grid(ctx);
-#if PD_HJ_ONE_TABLE
-  if (l.part_bits) {
-    // One table of 2^bits slots for all partitions, one build and one probe
-    // launch over the partitioned rows.  A key's home bucket is the top bits
-    // of the same hash whose top part_bits chose its partition, so the rows of
-    // partition q touch only slice q of the table: the slice being built or
-    // probed stays L2-resident, and no launch waits for a partition's tail.
-    p.boff = p.poff = nullptr;
-    p.tilebase = nullptr;
-    p.part_bits = 0;
-    p.part = 0;
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-      k_hj_clear<<<clear_grid, 256, 0, s>>>(p);
-    }
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_BUILD, s);
-      k_hj_build<<<build_grid, 256, 0, s>>>(p);
-    }
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_PROBE, s);
-      k_hj_probe<<<pgrid, HJ_THREADS, 0, s>>>(p);
-    }
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-      k_hj_count<<<1, 1, 0, s>>>(p.status, nullptr, 1, total_tiles_direct, p.epoch, p.d_count);
-    }
-    return pd_launch_status(ctx);
-  }
-#endif
-  for (uint32_t q = 0; q < parts; ++q) {
-    p.part = q;
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-      k_hj_clear<<<clear_grid, 256, 0, s>>>(p);
-    }
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_BUILD, s);
-      k_hj_build<<<build_grid, 256, 0, s>>>(p);
-    }
-    {
-      pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_PROBE, s);
-      k_hj_probe<<<pgrid, HJ_THREADS, 0, s>>>(p);
-    }
-  }
+  // Early launches pay where launches count (1e6 probe rows: 37.8 -> 34.3 us);
+  // in a large join the next kernel's waiting CTAs cost more than its launch
+  // (2^28 probe rows, 2^25 build rows: 6.00 -> 6.11 ms).
+  const bool early = a->size_probe < (1u << 24);
+  // One table of 2^bits slots, one build and one probe launch over the
+  // (partitioned) rows.  A key's home bucket is the top bits of the same hash
+  // whose top part_bits chose its partition, so the rows of partition q touch
+  // only slice q of the table: the slice being built or probed stays
+  // L2-resident, and no launch waits for a partition's tail.
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_hj_count<<<1, 1, 0, s>>>(p.status, p.tilebase, parts, total_tiles_direct, p.epoch, p.d_count);
+    PD_CHECK_CUDA(pd_launch_early(early, k_hj_clear, clear_grid, 256, 0, s, 1, p));
+  }
+  {
+    pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_BUILD, s);
+    PD_CHECK_CUDA(pd_launch_early(early, k_hj_build, build_grid, 256, 0, s, 1, p));
+  }
+  {
+    pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_PROBE, s);
+    PD_CHECK_CUDA(pd_launch_early(early, k_hj_probe, pgrid, HJ_THREADS, 0, s, 1, p));
   }
   return pd_launch_status(ctx);
 }
@@ -1279,11 +1182,11 @@ extern "C" int pimdal_hash_kernel(pimdal_ctx_t *ctx, const pimdal_hash_arguments
   PD_CHECK_CUDA(cudaMemsetAsync(a->table_ptr, 0, 32, s));
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_hj_clear<<<(unsigned)std::min<uint64_t>(pd_ceil_div(a->table_size, 512), ctx->sm_count * 8ull), 256, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_hj_clear, (unsigned)std::min<uint64_t>(pd_ceil_div(a->table_size, 512), ctx->sm_count * 8ull), 256, 0, s, 1, p));
   }
   if (a->size) {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_BUILD, s);
-    k_hj_build<<<ctx->sm_count * 8, 256, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_hj_build, ctx->sm_count * 8, 256, 0, s, 1, p));
   }
   return pd_launch_status(ctx);
 }
@@ -1326,11 +1229,7 @@ extern "C" int pimdal_hj_probe(pimdal_ctx_t *ctx, const pimdal_probe_arguments_t
   if (st) return st;
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_PROBE, s);
-    k_hj_probe<<<probe_grid(ctx), HJ_THREADS, 0, s>>>(p);
-  }
-  {
-    pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_hj_count<<<1, 1, 0, s>>>(p.status, nullptr, 1, tiles, p.epoch, p.d_count);
+    PD_CHECK_CUDA(pd_launch(k_hj_probe, probe_grid(ctx), HJ_THREADS, 0, s, 1, p));
   }
   return pd_launch_status(ctx);
 }
@@ -1510,6 +1409,7 @@ uint32_t sja_tables(uint32_t key_space) { return key_space <= SJA_WARP_KEYS ? SJ
 // dependent chain, and twice the warps of the former 4 CTAs per SM hide it
 // (a 6e7-row request 1.03 -> 0.61 ms).
 __global__ void __launch_bounds__(SJA_THREADS, 8) k_sja_aggregate(SjaParams p) {
+  pd_grid_dep();
   extern __shared__ __align__(16) unsigned long long sja_smem[];
   const uint32_t ks = p.key_space;
   const uint32_t tables = ks <= SJA_WARP_KEYS ? SJA_WARPS : 1;
@@ -1589,6 +1489,7 @@ __global__ void __launch_bounds__(1024) k_sja_emit(const unsigned long long *g_s
                                                    uint32_t *out_key, int64_t *out_sum,
                                                    int64_t *out_count, uint64_t cap,
                                                    uint64_t *t_count, uint32_t *d_error) {
+  pd_grid_dep();
   __shared__ uint32_t s_warp[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t base = 0;
@@ -1672,12 +1573,12 @@ extern "C" int pimdal_select_join_aggregate(pimdal_ctx_t *ctx,
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_FUSED, s);
     const size_t smem = 12ull * sja_tables(a->key_space) * a->key_space;
     const unsigned g = (unsigned)std::min<uint64_t>(pd_ceil_div(a->size, SJA_THREADS), ctx->sm_count * 8ull);
-    k_sja_aggregate<<<g, SJA_THREADS, smem, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_sja_aggregate, g, SJA_THREADS, smem, s, 1, p));
   }
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_sja_emit<<<1, 1024, 0, s>>>(p.g_sum, p.g_cnt, a->key_space, a->out_key, a->out_sum,
-                                  a->out_count, a->out_capacity, &d_result->t_count, ctx->d_error);
+    PD_CHECK_CUDA(pd_launch(k_sja_emit, 1, 1024, 0, s, 1, p.g_sum, p.g_cnt, a->key_space, a->out_key, a->out_sum,
+                                  a->out_count, a->out_capacity, &d_result->t_count, ctx->d_error));
   }
   return pd_launch_status(ctx);
 }

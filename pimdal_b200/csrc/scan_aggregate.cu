@@ -100,6 +100,7 @@ __device__ __forceinline__ void sa_load_rows(const SaCol &c, const uint32_t (&ro
 // latency of its dependent column loads, and 5 CTAs hide more of it than 4
 // at 64 registers (Q6 0.50 -> 0.43 ms, Q1 1.12 -> 0.98 ms on 6e7 rows).
 __global__ void __launch_bounds__(SA_THREADS, 5) k_sa_scan(SaParams p) {
+  pd_grid_dep();
   extern __shared__ __align__(16) unsigned long long sa_acc[];
   const int tid = threadIdx.x;
   const uint32_t nv = p.nexprs + 1;
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(SA_THREADS, 5) k_sa_scan(SaParams p) {
 __global__ void __launch_bounds__(1024) k_sa_emit(const unsigned long long *g_acc, uint32_t ks,
                                                   uint32_t nexprs, SaOut o, uint64_t *t_count,
                                                   uint32_t *d_error) {
+  pd_grid_dep();
   __shared__ uint32_t s_warp[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t nv = nexprs + 1;
@@ -402,7 +404,7 @@ extern "C" int pimdal_select_aggregate(pimdal_ctx_t *ctx,
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>(want, (uint64_t)per_sm * ctx->sm_count));
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_SCAN_AGG, s);
-    k_sa_scan<<<grid, SA_THREADS, smem, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_sa_scan, grid, SA_THREADS, smem, s, 1, p));
   }
   SaOut o{};
   o.key = a->out_key;
@@ -411,8 +413,8 @@ extern "C" int pimdal_select_aggregate(pimdal_ctx_t *ctx,
   o.cap = a->out_capacity;
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_sa_emit<<<1, 1024, 0, s>>>(p.g_acc, a->key_space, a->n_exprs, o, &d_result->t_count,
-                                 ctx->d_error);
+    PD_CHECK_CUDA(pd_launch(k_sa_emit, 1, 1024, 0, s, 1, p.g_acc, a->key_space, a->n_exprs, o, &d_result->t_count,
+                                 ctx->d_error));
   }
   return pd_launch_status(ctx);
 }

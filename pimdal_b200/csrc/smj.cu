@@ -53,7 +53,7 @@ struct MergeParams {
   uint64_t *bounds;  // [2 * tiles]: inner range per tile
   uint64_t *status;
   uint32_t epoch;
-  uint32_t *claim;   // tile counter (zeroed by the host before the launch)
+  uint32_t *claim;   // tile counter (zeroed by k_smj_bounds)
   uint32_t *d_error;
   uint64_t *d_count;
 };
@@ -73,7 +73,9 @@ __device__ __forceinline__ uint64_t gsearch(const uint32_t *key, uint64_t lo, ui
 }
 
 __global__ void __launch_bounds__(256) k_smj_bounds(MergeParams p) {
+  pd_grid_dep();
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) *p.claim = 0;  // the merge's tile counter
   if (t >= p.tiles) return;
   uint64_t o0 = t * MJ_TILE, o1 = min(p.no, o0 + MJ_TILE);
   uint32_t kf = ord(p.okey[o0], p.flip), kl = ord(p.okey[o1 - 1], p.flip);
@@ -96,6 +98,7 @@ __device__ __forceinline__ uint32_t ssearch(const uint32_t *k, uint32_t lo, uint
 // 5 CTAs per SM (48 registers; 41 KB of shared memory each): measured 10%
 // faster than 4 at 64 registers, the extra warps hiding the tile's loads.
 __global__ void __launch_bounds__(MJ_THREADS, 5) k_smj_merge(MergeParams p) {
+  pd_grid_dep();
   __shared__ uint32_t s_ik[MJ_INNER_CAP];
   __shared__ uint32_t s_ip[MJ_INNER_CAP];
   __shared__ uint32_t s_oo[MJ_OUT_CAP];  // staged output of the tile
@@ -261,14 +264,13 @@ int launch_merge(pimdal_ctx *ctx, MergeParams &p, cudaStream_t s) {
   if (st) return st;
   p.status = ctx->d_status;
   p.d_error = ctx->d_error;
-  PD_CHECK_CUDA(cudaMemsetAsync(p.claim, 0, sizeof(uint32_t), s));
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_smj_bounds<<<(unsigned)pd_ceil_div(p.tiles, 256), 256, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_smj_bounds, (unsigned)pd_ceil_div(p.tiles, 256), 256, 0, s, 1, p));
   }
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_SMJ_MERGE, s);
-    k_smj_merge<<<(unsigned)p.tiles, MJ_THREADS, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(k_smj_merge, (unsigned)p.tiles, MJ_THREADS, 0, s, 1, p));
   }
   return pd_launch_status(ctx);
 }

@@ -12,18 +12,24 @@
 // B200 design (HBM-bound, no tensor cores):
 //  1. k_sort_hist: one read of the keys builds the 256-bin histograms of all
 //     digit positions (warp-private shared-memory counters).
-//  2. k_sort_plan (one CTA): exclusive scans of the histograms; a pass whose
-//     digit is the same for every key (count == n) is skipped; buffers are
-//     routed so the last active pass writes the caller's output.  Computed on
-//     the device, so the whole sort is stream-ordered and capturable.
+//  2. the last CTA of k_sort_hist makes the plan: exclusive scans of the
+//     histograms; a pass whose digit is the same for every key (count == n) is
+//     skipped; buffers are routed so the last active pass writes the caller's
+//     output.  Computed on the device, so the whole sort is stream-ordered and
+//     capturable.
 //  3. k_sort_pass, once per digit: a CTA takes the next tile of RS_TILE keys
 //     (atomic tile counter, so tiles are processed in input order), counts
 //     its digits and publishes the counts early, ranks keys per warp
 //     (shared-memory lane masks group the lanes of one digit), resolves the
 //     digits' global offsets with a per-digit decoupled look-back, stages the
 //     tile in shared memory in digit order and writes each digit run
-//     contiguously.
+//     contiguously.  Inputs that do not fill the GPU with full tiles take
+//     smaller ones.
+//  Up to SS_MAX_N pairs are sorted by one cluster in one launch instead
+//  (k_sort_cluster).
 #include <algorithm>
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 
@@ -46,19 +52,32 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 #define PD_RS_WFULL 1  // 1: full tiles write their staged keys in a fully unrolled loop
 #endif
 constexpr int RS_ITEMS = PD_RS_ITEMS;
-constexpr int RS_WARP_TILE = 32 * RS_ITEMS;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+#ifndef PD_RS_SMALL_ITEMS
+#define PD_RS_SMALL_ITEMS 8
+#endif
+constexpr int RS_SMALL_ITEMS = PD_RS_SMALL_ITEMS;  // keys per thread where full tiles leave SMs idle
 constexpr int RS_MIN_CTAS = PD_RS_MIN_CTAS;
 static_assert(RS_ITEMS % 2 == 0 && RS_TILE <= 65536, "16-bit packed staged positions");
+static_assert(RS_SMALL_ITEMS % 2 == 0 && RS_SMALL_ITEMS <= RS_ITEMS, "small tiles");
 constexpr int RS_RADIX_BITS = 8;
 constexpr int RS_RADIX = 1 << RS_RADIX_BITS;       // 256 (== RS_THREADS)
 constexpr int RS_MAX_PASSES = 4;
+// Look-back word of a (tile, digit): [flag:2][count:30].  With small tiles it is
+// [flag:2][pass:2][count:28] and all passes share one array of words (a word
+// of another pass reads as not there yet), so that the smaller tiles need no
+// more scratch.
 constexpr uint32_t RS_FLAG_AGG = 1u << 30, RS_FLAG_INC = 2u << 30, RS_COUNT_MASK = (1u << 30) - 1;
+constexpr uint32_t RS_SHARED_MASK = (1u << 28) - 1;
 static_assert(RS_RADIX == RS_THREADS, "one thread per digit");
 // The atomicOr masks (two per warp and digit) borrow the staging buffer
-// during the ranking; it must hold them even for keys alone.
+// during the ranking.
 constexpr int RS_MATCH_WORDS = 2 * RS_WARPS * RS_RADIX;
-static_assert(PD_RS_MATCH == 0 || RS_MATCH_WORDS <= RS_TILE, "match masks fit the key staging");
+static_assert(RS_MATCH_WORDS * 4 % (16 * RS_THREADS) == 0, "masks cleared in 16-byte stores");
+constexpr size_t rs_smem_bytes(int items, bool vals) {
+  const size_t stage = (size_t)(vals ? 8 : 4) * RS_THREADS * items, masks = 4 * RS_MATCH_WORDS;
+  return stage > masks ? stage : masks;
+}
 
 enum : uint32_t { BUF_IN = 0, BUF_OUT = 1, BUF_ALT = 2 };
 
@@ -96,8 +115,8 @@ struct SortParams {
   uint32_t *hist;       // [RS_MAX_PASSES][RS_RADIX]
   uint32_t *offsets;    // [RS_MAX_PASSES][RS_RADIX]
   SortPlan *plan;
-  uint32_t *status;     // [RS_MAX_PASSES][tiles][RS_RADIX]
-  uint32_t *counters;   // [RS_MAX_PASSES]
+  uint32_t *status;     // [passes, or 1 with small tiles][tiles][RS_RADIX]
+  uint32_t *counters;   // [RS_MAX_PASSES], then k_sort_hist's finished CTAs
   uint64_t tiles;
   uint32_t *d_error;
 };
@@ -117,9 +136,70 @@ __device__ __forceinline__ uint32_t hist_xform(uint32_t k, uint32_t flip) {
   return k ^ flip;
 }
 
+// Block-wide exclusive scan of one value per thread (RS_THREADS threads).
+__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s_warp,
+                                                         uint32_t *total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  uint32_t wpre = 0, tot = 0;
+#pragma unroll
+  for (int w = 0; w < RS_WARPS; ++w) {
+    uint32_t x = s_warp[w];
+    if (w < warp) wpre += x;
+    tot += x;
+  }
+  __syncthreads();
+  if (total) *total = tot;
+  return wpre + inc - v;
+}
+
+// Exclusive scans of the finished histograms and the passes' routing (one CTA;
+// sh: RS_WARPS + RS_MAX_PASSES words).
+__device__ __forceinline__ void sort_plan(const SortParams &p, uint32_t *sh) {
+  uint32_t *s_warp = sh, *s_trivial = sh + RS_WARPS;
+  const int d = threadIdx.x;
+  const uint64_t n = sort_n(p);
+  if (d < RS_MAX_PASSES) s_trivial[d] = 0;
+  __syncthreads();
+  for (uint32_t q = 0; q < p.npasses; ++q) {
+    const uint32_t c = __ldcg(&p.hist[q * RS_RADIX + d]);
+    if ((uint64_t)c == n) s_trivial[q] = 1;
+    p.offsets[q * RS_RADIX + d] = block_exclusive_scan(c, s_warp, nullptr);
+  }
+  __syncthreads();
+  if (d == 0) {
+    SortPlan pl{};
+    uint32_t m = 0;
+    for (uint32_t q = 0; q < p.npasses; ++q) {
+      pl.active[q] = !s_trivial[q];
+      m += pl.active[q];
+    }
+    pl.n_active = m;
+    uint32_t j = 0, prev = BUF_IN;
+    for (uint32_t q = 0; q < p.npasses; ++q) {
+      if (!pl.active[q]) continue;
+      ++j;
+      pl.src[q] = prev;
+      pl.dst[q] = ((m - j) % 2 == 0) ? BUF_OUT : BUF_ALT;
+      pl.first[q] = (j == 1);
+      prev = pl.dst[q];
+    }
+    *p.plan = pl;
+  }
+}
+
 template <int KEY_MODE>
 __global__ void __launch_bounds__(RS_THREADS) k_sort_hist(SortParams p) {
+  pd_grid_dep();
   __shared__ uint32_t sh[RS_WARPS][RS_MAX_PASSES][RS_RADIX];
+  __shared__ bool s_last;
   const int tid = threadIdx.x, warp = tid >> 5;
   for (int i = tid; i < RS_WARPS * RS_MAX_PASSES * RS_RADIX; i += RS_THREADS)
     (&sh[0][0][0])[i] = 0;
@@ -187,70 +267,20 @@ __global__ void __launch_bounds__(RS_THREADS) k_sort_hist(SortParams p) {
     for (int w = 0; w < RS_WARPS; ++w) s += sh[w][q][tid];
     if (s) atomicAdd(&p.hist[q * RS_RADIX + tid], s);
   }
+  // the last CTA to add its counts makes the plan
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&p.counters[RS_MAX_PASSES], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  sort_plan(p, &sh[0][0][0]);
 }
 
-// Block-wide exclusive scan of one value per thread (RS_THREADS threads).
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s_warp,
-                                                         uint32_t *total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) s_warp[warp] = inc;
-  __syncthreads();
-  uint32_t wpre = 0, tot = 0;
-#pragma unroll
-  for (int w = 0; w < RS_WARPS; ++w) {
-    uint32_t x = s_warp[w];
-    if (w < warp) wpre += x;
-    tot += x;
-  }
-  __syncthreads();
-  if (total) *total = tot;
-  return wpre + inc - v;
-}
-
-// -------------------------------------------------------------------- plan
-__global__ void __launch_bounds__(RS_THREADS) k_sort_plan(SortParams p) {
-  __shared__ uint32_t s_warp[RS_WARPS];
-  __shared__ uint32_t s_trivial[RS_MAX_PASSES];
-  const int d = threadIdx.x;
-  const uint64_t n = sort_n(p);
-  if (d < RS_MAX_PASSES) s_trivial[d] = 0;
-  __syncthreads();
-  for (uint32_t q = 0; q < p.npasses; ++q) {
-    uint32_t c = p.hist[q * RS_RADIX + d];
-    if ((uint64_t)c == n) s_trivial[q] = 1;
-    p.offsets[q * RS_RADIX + d] = block_exclusive_scan(c, s_warp, nullptr);
-  }
-  __syncthreads();
-  if (d == 0) {
-    SortPlan pl{};
-    uint32_t m = 0;
-    for (uint32_t q = 0; q < p.npasses; ++q) {
-      pl.active[q] = !s_trivial[q];
-      m += pl.active[q];
-    }
-    pl.n_active = m;
-    uint32_t j = 0, prev = BUF_IN;
-    for (uint32_t q = 0; q < p.npasses; ++q) {
-      if (!pl.active[q]) continue;
-      ++j;
-      pl.src[q] = prev;
-      pl.dst[q] = ((m - j) % 2 == 0) ? BUF_OUT : BUF_ALT;
-      pl.first[q] = (j == 1);
-      prev = pl.dst[q];
-    }
-    *p.plan = pl;
-  }
-}
-
-// No active pass (all keys share every digit, or n small): copy in -> out.
-__global__ void __launch_bounds__(RS_THREADS) k_sort_copy(SortParams p) {
-  if (p.plan->n_active != 0) return;
+// No active pass (all keys share every digit): copy in -> out, in pass 0 of a
+// sort by small tiles, in a launch of its own otherwise (the full tiles' pass
+// has no register to spare for it: 1% slower).
+__device__ __forceinline__ void sort_copy(const SortParams &p) {
   const uint64_t stride = (uint64_t)gridDim.x * RS_THREADS;
   const uint64_t n = sort_n(p);
   for (uint64_t i = (uint64_t)blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += stride) {
@@ -273,6 +303,11 @@ __global__ void __launch_bounds__(RS_THREADS) k_sort_copy(SortParams p) {
   }
 }
 
+__global__ void __launch_bounds__(RS_THREADS) k_sort_copy(SortParams p) {
+  pd_grid_dep();
+  if (p.plan->n_active == 0) sort_copy(p);
+}
+
 // ------------------------------------------------------------ onesweep pass
 template <int KEY_MODE>
 __device__ __forceinline__ uint32_t sort_xform(uint32_t k, uint32_t flip) {
@@ -291,9 +326,10 @@ __device__ __forceinline__ uint32_t sort_xform(uint32_t k, uint32_t flip) {
 #ifndef PD_RS_LOOKBACK
 #define PD_RS_LOOKBACK 4  // predecessor words per look-back round of the digit pass
 #endif
-template <int RS_LOOKBACK>
+template <int RS_LOOKBACK, bool TAGGED>
 __device__ __forceinline__ uint32_t rs_lookback(uint32_t *st, uint64_t tile, uint32_t count,
-                                                uint32_t *d_error) {
+                                                uint32_t tag, uint32_t *d_error) {
+  constexpr uint32_t count_mask = TAGGED ? RS_SHARED_MASK : RS_COUNT_MASK;
   uint32_t excl = 0;
   int64_t t = (int64_t)tile - 1;
   uint32_t spins = 0;
@@ -302,18 +338,18 @@ __device__ __forceinline__ uint32_t rs_lookback(uint32_t *st, uint64_t tile, uin
     uint32_t w[RS_LOOKBACK];
 #pragma unroll
     for (int i = 0; i < RS_LOOKBACK; ++i)
-      w[i] = (t - i >= 0) ? pd_load_relaxed_u32(st + (uint64_t)(t - i) * RS_RADIX) : RS_FLAG_INC;
+      w[i] = (t - i >= 0) ? pd_load_relaxed_u32(st + (uint64_t)(t - i) * RS_RADIX) : RS_FLAG_INC | tag;
     int used = 0;
     bool done = false, stalled = false;
 #pragma unroll
     for (int i = 0; i < RS_LOOKBACK; ++i) {
       if (done || stalled) continue;
-      const uint32_t flag = w[i] & ~RS_COUNT_MASK;
-      if (flag == 0) {
+      const uint32_t flag = TAGGED ? (w[i] & ~count_mask) ^ tag : w[i] & ~count_mask;
+      if (TAGGED ? flag != RS_FLAG_AGG && flag != RS_FLAG_INC : flag == 0) {
         stalled = true;
         continue;
       }
-      excl += w[i] & RS_COUNT_MASK;
+      excl += w[i] & count_mask;
       ++used;
       if (flag == RS_FLAG_INC) done = true;
     }
@@ -324,7 +360,7 @@ __device__ __forceinline__ uint32_t rs_lookback(uint32_t *st, uint64_t tile, uin
       __nanosleep(spins < 8 ? 64 : 256);
     }
   }
-  pd_store_relaxed_u32(st + tile * RS_RADIX, RS_FLAG_INC | ((excl + count) & RS_COUNT_MASK));
+  pd_store_relaxed_u32(st + tile * RS_RADIX, RS_FLAG_INC | tag | ((excl + count) & count_mask));
   return excl;
 }
 
@@ -343,9 +379,11 @@ __device__ __forceinline__ unsigned match_digit(uint32_t d, unsigned members) {
 
 // One digit pass.  FULL tiles take a path without bounds checks; indices
 // inside a tile are 32-bit; the digit is (xform(key) >> shift) & mask.
-template <bool HAS_VALS, int KEY_MODE>
+template <bool HAS_VALS, int KEY_MODE, int ITEMS, int LOOKBACK>
 __global__ void __launch_bounds__(RS_THREADS, RS_MIN_CTAS)
 k_sort_pass(SortParams p, uint32_t pass, uint32_t shift, uint32_t mask) {
+  constexpr int RS_ITEMS = ITEMS, RS_TILE = RS_THREADS * ITEMS, RS_WARP_TILE = 32 * ITEMS;
+  pd_grid_dep();
   // the tile staged in digit order: (key, value) words, or keys alone
   extern __shared__ __align__(16) uint2 rs_stage[];  // RS_TILE (key, value) words or keys
   uint2 *s_kv = rs_stage;
@@ -356,11 +394,16 @@ k_sort_pass(SortParams p, uint32_t pass, uint32_t shift, uint32_t mask) {
   __shared__ uint32_t s_warp[RS_WARPS];
   __shared__ uint32_t s_tile;
 
+  constexpr bool SMALL = ITEMS == RS_SMALL_ITEMS;
   const SortPlan *plan = p.plan;
-  if (!plan->active[pass]) return;
+  if (!plan->active[pass]) {
+    if (SMALL && pass == 0 && plan->n_active == 0) sort_copy(p);
+    return;
+  }
   const uint32_t src = plan->src[pass], dst = plan->dst[pass];
   const bool first = plan->first[pass] != 0;
   const uint32_t flip = p.flip;
+  const uint32_t tag = SMALL ? pass << 28 : 0u;
   auto dig = [&](uint32_t k) { return (sort_xform<KEY_MODE>(k, flip) >> shift) & mask; };
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -442,9 +485,9 @@ k_sort_pass(SortParams p, uint32_t pass, uint32_t shift, uint32_t mask) {
     run += t;
   }
   const uint32_t count = run;
-  uint32_t *st = p.status + ((uint64_t)pass * p.tiles) * RS_RADIX + d;
-  if (tile == 0) pd_store_relaxed_u32(st, RS_FLAG_INC | count);
-  else pd_store_relaxed_u32(st + tile * RS_RADIX, RS_FLAG_AGG | count);
+  uint32_t *st = p.status + (SMALL ? 0ull : (uint64_t)pass * p.tiles) * RS_RADIX + d;
+  if (tile == 0) pd_store_relaxed_u32(st, RS_FLAG_INC | tag | count);
+  else pd_store_relaxed_u32(st + tile * RS_RADIX, RS_FLAG_AGG | tag | count);
   const uint32_t dstart = block_exclusive_scan(count, s_warp, nullptr);
   // each warp's first position of digit d in the staged tile seeds its
   // running counter, so the ranking below yields staged positions
@@ -527,7 +570,7 @@ k_sort_pass(SortParams p, uint32_t pass, uint32_t shift, uint32_t mask) {
 
   // The digit's global offset.  (Looking back before the ranking instead,
   // to publish the inclusive counts earlier, was measured no faster.)
-  const uint32_t excl = tile > 0 ? rs_lookback<PD_RS_LOOKBACK>(st, tile, count, p.d_error) : 0u;
+  const uint32_t excl = tile > 0 ? rs_lookback<LOOKBACK, SMALL>(st, tile, count, tag, p.d_error) : 0u;
   s_gdelta[d] = (int32_t)(p.offsets[pass * RS_RADIX + d] + excl) - (int32_t)dstart;
   __syncthreads();
 
@@ -565,6 +608,233 @@ k_sort_pass(SortParams p, uint32_t pass, uint32_t shift, uint32_t mask) {
 #pragma unroll 4
   for (uint32_t i = tid; i < tile_n; i += RS_THREADS) put(i);
   }
+}
+
+// ------------------------------------------------------------- short inputs
+// Up to SS_CLUSTER * SS_TILE pairs: the whole sort in one launch of one
+// thread-block cluster.  Every pair lives in the registers of the thread that
+// holds its position; a pass ranks the CTA's pairs (the same lane masks and
+// warp counters as the digit pass), exchanges the CTAs' digit counts through
+// distributed shared memory and scatters the pairs straight into the buffer of
+// the CTA that owns their new position.  A pass costs two cluster barriers
+// instead of a launch, a histogram read and a look-back chain through L2: such
+// inputs leave most of the GPU idle either way, and what they paid was eight
+// launches (1000 pairs 65 -> 15 us, 8000 pairs 75 -> 21 us).  A CTA ranks about
+// one pair per two cycles (shared-memory wavefronts), so above 32768 pairs
+// many SMs win (50,000 pairs: 56 us by 8 CTAs, 45 us by small tiles).
+constexpr int SS_THREADS = 1024;
+constexpr int SS_WARPS = SS_THREADS / 32;
+constexpr int SS_ITEMS = 4;
+constexpr int SS_TILE = SS_THREADS * SS_ITEMS;  // pairs of a CTA
+constexpr int SS_CLUSTER = 8;                   // CTAs (the largest portable cluster)
+constexpr int SS_PARTS = SS_THREADS / RS_RADIX; // threads per digit in the count steps
+#ifndef PD_SS_MIN_CHUNK
+#define PD_SS_MIN_CHUNK 1024
+#endif
+constexpr uint64_t SS_MIN_CHUNK = PD_SS_MIN_CHUNK;  // pairs per CTA before another joins the cluster
+constexpr uint64_t SS_MAX_N = (uint64_t)SS_CLUSTER * SS_TILE;
+constexpr int SS_MASK_WORDS = 2 * SS_WARPS * RS_RADIX;  // two mask sets per warp
+static_assert(SS_CLUSTER % SS_PARTS == 0 && SS_WARPS % SS_PARTS == 0, "count steps");
+constexpr size_t ss_smem_bytes(bool vals) {
+  return (size_t)(vals ? 8 : 4) * SS_TILE + 4 * SS_MASK_WORDS + 2 * SS_WARPS * RS_RADIX;
+}
+
+template <bool HAS_VALS>
+__global__ void __launch_bounds__(SS_THREADS, 1) k_sort_cluster(SortParams p) {
+  pd_grid_trigger();
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char ss_smem[];
+  uint2 *s_kv = reinterpret_cast<uint2 *>(ss_smem);
+  uint32_t *s_k = reinterpret_cast<uint32_t *>(ss_smem);
+  uint32_t *s_mask = reinterpret_cast<uint32_t *>(ss_smem + (HAS_VALS ? 8 : 4) * SS_TILE);
+  uint16_t *s_wcnt = reinterpret_cast<uint16_t *>(s_mask + SS_MASK_WORDS);  // [warp][digit]
+  __shared__ uint32_t s_count[2][RS_RADIX];         // this CTA's digit counts, by pass parity
+  __shared__ uint32_t s_sum[SS_PARTS][RS_RADIX], s_before[SS_PARTS][RS_RADIX];
+  __shared__ uint32_t s_base[RS_RADIX];             // first position of this CTA's pairs of a digit
+  __shared__ uint32_t s_warp[RS_WARPS];
+  __shared__ uint32_t s_trivial;
+
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t ctas = cluster.num_blocks(), cta = cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int d = tid & (RS_RADIX - 1), part = tid / RS_RADIX;  // digit and share in the count steps
+  // lane masks to zero; the ranking leaves them so
+#pragma unroll
+  for (int j = 0; j < SS_MASK_WORDS / (4 * SS_THREADS); ++j)
+    reinterpret_cast<uint4 *>(s_mask)[tid + j * SS_THREADS] = make_uint4(0, 0, 0, 0);
+  pd_grid_wait();
+  const uint32_t n = (uint32_t)sort_n(p);
+  const uint32_t chunk = (n + ctas - 1) / ctas;     // positions of a CTA
+  const uint32_t items = (chunk + SS_THREADS - 1) / SS_THREADS;
+  const uint32_t first = cta * chunk;
+  const uint32_t rows = first < n ? min(chunk, n - first) : 0u;
+  // position / chunk: exact for positions below 2^17 and chunks up to 2^14
+  const uint32_t inv = chunk ? (uint32_t)(0x100000000ull / chunk) + (chunk > 1) : 0u;
+  const uint32_t flip = p.flip;
+
+  // item k of this thread is the CTA's position w0 + 32 k
+  const uint32_t w0 = (uint32_t)warp * 32u * items + lane;
+  uint32_t key[SS_ITEMS], val[HAS_VALS ? SS_ITEMS : 1];
+  const long long pmin = p.pay64 && !p.in_ptr ? *p.pay_min : 0;
+#pragma unroll
+  for (int k = 0; k < SS_ITEMS; ++k) {
+    key[k] = 0;
+    if (HAS_VALS) val[k] = 0;
+    if (k < (int)items && w0 + 32u * k < rows) {
+      const uint32_t i = first + w0 + 32u * k;
+      if (p.pairs) {
+        const uint2 e = reinterpret_cast<const uint2 *>(p.in)[i];
+        key[k] = e.x;
+        if (HAS_VALS) val[k] = e.y;
+      } else {
+        key[k] = reinterpret_cast<const uint32_t *>(p.in)[i];
+        if (HAS_VALS)
+          val[k] = p.in_ptr ? p.in_ptr[i] : p.pay64 ? (uint32_t)(p.pay64[i] - pmin) : (uint32_t)(p.ptr_base + i);
+      }
+    }
+  }
+
+  const uint32_t lt = (1u << lane) - 1u, lanebit = 1u << lane;
+  for (uint32_t q = 0; q < p.npasses; ++q) {
+    const uint32_t shift = p.begin_bit + q * RS_RADIX_BITS;
+    const uint32_t mask = (1u << min((uint32_t)RS_RADIX_BITS, p.end_bit - shift)) - 1u;
+    auto dig = [&](uint32_t x) { return ((x ^ flip) >> shift) & mask; };
+#pragma unroll
+    for (int j = 0; j < SS_WARPS * RS_RADIX / (8 * SS_THREADS); ++j)
+      reinterpret_cast<uint4 *>(s_wcnt)[tid + j * SS_THREADS] = make_uint4(0, 0, 0, 0);
+    if (tid == 0) s_trivial = 0;
+    __syncthreads();
+    // rank within (warp, digit), in position order: as in the digit pass
+    uint32_t rank2[SS_ITEMS / 2];
+    uint32_t *mbase = s_mask + warp * 2 * RS_RADIX;
+    uint16_t *wcnt = s_wcnt + warp * RS_RADIX;
+#pragma unroll
+    for (int k = 0; k < SS_ITEMS; ++k) {
+      if (!(k & 1)) rank2[k >> 1] = 0;
+      if (k < (int)items) {
+        const bool valid = w0 + 32u * k < rows;
+        const uint32_t dk = dig(key[k]);
+        uint32_t *mb = mbase + (k & 1) * RS_RADIX;
+        if (valid) atomicOr(&mb[dk], lanebit);
+        __syncwarp();
+        const unsigned peers = valid ? mb[dk] : lanebit;
+        const int leader = 31 - __clz(peers);
+        uint32_t old = 0;
+        if (valid && lane == leader) old = wcnt[dk];
+        old = __shfl_sync(0xffffffffu, old, leader);
+        if (valid && lane == leader) {
+          wcnt[dk] = (uint16_t)(old + __popc(peers));
+          mb[dk] = 0;
+        }
+        rank2[k >> 1] |= (old + __popc(peers & lt)) << (16 * (k & 1));
+      }
+    }
+    __syncthreads();
+    // digit counts of the CTA; the warps' counts become their first ranks
+    {
+      constexpr int W = SS_WARPS / SS_PARTS;
+      uint32_t c[W], t = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        c[w] = s_wcnt[(part * W + w) * RS_RADIX + d];
+        t += c[w];
+      }
+      s_sum[part][d] = t;
+      __syncthreads();
+      uint32_t at = 0;
+#pragma unroll
+      for (int x = 0; x < SS_PARTS - 1; ++x)
+        if (x < part) at += s_sum[x][d];
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        s_wcnt[(part * W + w) * RS_RADIX + d] = (uint16_t)at;
+        at += c[w];
+      }
+      if (part == SS_PARTS - 1) s_count[q & 1][d] = at;
+    }
+    cluster.sync();
+    // all CTAs' counts: digit totals and those of the CTAs before this one
+    {
+      uint32_t total = 0, before = 0;
+#pragma unroll
+      for (int j = 0; j < SS_CLUSTER / SS_PARTS; ++j) {
+        const uint32_t c = part + j * SS_PARTS;
+        if (c < ctas) {
+          const uint32_t x = cluster.map_shared_rank(&s_count[q & 1][0], c)[d];
+          total += x;
+          if (c < cta) before += x;
+        }
+      }
+      s_sum[part][d] = total;
+      s_before[part][d] = before;
+    }
+    __syncthreads();
+    uint32_t total = 0, before = 0, inc = 0;
+    if (tid < RS_RADIX) {
+#pragma unroll
+      for (int x = 0; x < SS_PARTS; ++x) {
+        total += s_sum[x][d];
+        before += s_before[x][d];
+      }
+      if (total == n) s_trivial = 1;
+      inc = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (lane == 31) s_warp[warp] = inc;
+    }
+    __syncthreads();
+    if (tid < RS_RADIX) {
+      uint32_t pre = 0;
+#pragma unroll
+      for (int w = 0; w < RS_WARPS; ++w)
+        if (w < warp) pre += s_warp[w];
+      s_base[d] = pre + inc - total + before;
+    }
+    __syncthreads();
+    if (s_trivial) {  // every key has the same digit: nothing moves
+      __syncthreads();  // s_trivial is cleared by the next pass
+      continue;
+    }
+#pragma unroll
+    for (int k = 0; k < SS_ITEMS; ++k) {
+      if (k < (int)items && w0 + 32u * k < rows) {
+        const uint32_t dk = dig(key[k]);
+        const uint32_t g = s_base[dk] + wcnt[dk] + ((rank2[k >> 1] >> (16 * (k & 1))) & 0xFFFFu);
+        const uint32_t c = chunk > 1 ? __umulhi(g, inv) : g, o = g - c * chunk;
+        if (HAS_VALS) cluster.map_shared_rank(s_kv, c)[o] = make_uint2(key[k], val[k]);
+        else cluster.map_shared_rank(s_k, c)[o] = key[k];
+      }
+    }
+    cluster.sync();
+#pragma unroll
+    for (int k = 0; k < SS_ITEMS; ++k) {
+      if (k < (int)items && w0 + 32u * k < rows) {
+        if (HAS_VALS) {
+          const uint2 e = s_kv[w0 + 32u * k];
+          key[k] = e.x;
+          val[k] = e.y;
+        } else {
+          key[k] = s_k[w0 + 32u * k];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < SS_ITEMS; ++k) {
+    if (k < (int)items && w0 + 32u * k < rows) {
+      const uint32_t i = first + w0 + 32u * k;
+      if (p.pairs) {
+        if (HAS_VALS) reinterpret_cast<uint2 *>(p.out)[i] = make_uint2(key[k], val[k]);
+      } else {
+        reinterpret_cast<uint32_t *>(p.out)[i] = key[k];
+        if (HAS_VALS) p.out_ptr[i] = val[k];
+      }
+    }
+  }
+  cluster.sync();  // no CTA leaves while another may still read its counts
 }
 
 // ------------------------------------------------- small-radix partition pass
@@ -614,6 +884,7 @@ __device__ __forceinline__ void prefetch_l2(const void *ptr) {
 template <int BITS, int VAL, int KEY_MODE>
 __global__ void __launch_bounds__(RS_THREADS, 3)
 k_part_pass(SortParams p, uint32_t pass, uint32_t shift) {
+  pd_grid_dep();
   using S = PartShape<BITS>;
   constexpr bool HAS_VALS = VAL == PV_U32;
   constexpr bool V64 = VAL == PV_U64;
@@ -762,7 +1033,7 @@ k_part_pass(SortParams p, uint32_t pass, uint32_t shift) {
       pd_store_relaxed_u32(st, RS_FLAG_INC | count);
     } else {
       pd_store_relaxed_u32(st + tile * RS_RADIX, RS_FLAG_AGG | count);
-      ex = rs_lookback<8>(st, tile, count, p.d_error);
+      ex = rs_lookback<8, false>(st, tile, count, 0u, p.d_error);
     }
     s_gdelta[d] = (int32_t)(p.offsets[pass * RS_RADIX + d] + ex) - (int32_t)s_dstart[d];
   }
@@ -853,11 +1124,18 @@ PartKernel pick_part(uint32_t bits, int val, int key_mode) {
 }
 
 using PassKernel = void (*)(SortParams, uint32_t, uint32_t, uint32_t);
-PassKernel pick_pass(bool vals, int key_mode) {
-  if (key_mode == PD_KEY_HASH0) return vals ? k_sort_pass<true, PD_KEY_HASH0> : k_sort_pass<false, PD_KEY_HASH0>;
+template <bool VALS, int KEY_MODE>
+PassKernel pick_pass_items(bool small) {
+  // few tiles all start at once, so each looks back over more of them per round
+  return small ? k_sort_pass<VALS, KEY_MODE, RS_SMALL_ITEMS, 16>
+               : k_sort_pass<VALS, KEY_MODE, RS_ITEMS, PD_RS_LOOKBACK>;
+}
+PassKernel pick_pass(bool vals, int key_mode, bool small) {
+  if (key_mode == PD_KEY_HASH0)
+    return vals ? pick_pass_items<true, PD_KEY_HASH0>(small) : pick_pass_items<false, PD_KEY_HASH0>(small);
   if (key_mode == PD_KEY_MULHASH)
-    return vals ? k_sort_pass<true, PD_KEY_MULHASH> : k_sort_pass<false, PD_KEY_MULHASH>;
-  return vals ? k_sort_pass<true, PD_KEY_PLAIN> : k_sort_pass<false, PD_KEY_PLAIN>;
+    return vals ? pick_pass_items<true, PD_KEY_MULHASH>(small) : pick_pass_items<false, PD_KEY_MULHASH>(small);
+  return vals ? pick_pass_items<true, PD_KEY_PLAIN>(small) : pick_pass_items<false, PD_KEY_PLAIN>(small);
 }
 
 struct SortLayout {
@@ -865,7 +1143,16 @@ struct SortLayout {
       off_alt_v64, total, memset_bytes;
   uint64_t tiles;
   uint32_t npasses;
+  bool small;   // tiles of RS_SMALL_ITEMS keys per thread
 };
+
+// Below this many keys, tiles of 2048: full tiles of 5120 leave most of the GPU's
+// 444 resident CTAs without one.  (100,003 pairs 51 against 63 us, 400,000
+// pairs 64 us either way, 1,000,000 pairs 93 against 82 us.)
+#ifndef PD_RS_SMALL_N
+#define PD_RS_SMALL_N (3u << 17)
+#endif
+constexpr uint64_t RS_SMALL_N = PD_RS_SMALL_N;
 
 // dbits: digit width of each pass (8 for a sort; at most 6 for a partition,
 // which may also carry 64-bit values, v64).
@@ -875,11 +1162,15 @@ bool sort_layout(const pimdal_sort_arguments_t *a, SortLayout *l, uint32_t dbits
   if (b >= e || e > 32 || dbits == 0 || dbits > RS_RADIX_BITS) return false;
   l->npasses = (e - b + dbits - 1) / dbits;
   if (l->npasses > RS_MAX_PASSES) return false;
-  l->tiles = pd_ceil_div(a->nr_elements ? a->nr_elements : 1, RS_TILE);
+  const uint64_t n = a->nr_elements ? a->nr_elements : 1;
+  // (a partition's passes keep full tiles)
+  l->small = n < RS_SMALL_N && dbits == RS_RADIX_BITS;
+  l->tiles = pd_ceil_div(n, (uint64_t)RS_THREADS * (l->small ? RS_SMALL_ITEMS : RS_ITEMS));
   size_t o = 0;
   l->off_counters = o; o += 256;
   l->off_hist = o; o += sizeof(uint32_t) * RS_MAX_PASSES * RS_RADIX;
-  l->off_status = o; o += pd_align_up(sizeof(uint32_t) * RS_MAX_PASSES * l->tiles * RS_RADIX, 256);
+  l->off_status = o; o += pd_align_up(
+      sizeof(uint32_t) * (l->small ? 1 : RS_MAX_PASSES) * l->tiles * RS_RADIX, 256);
   l->memset_bytes = o;
   l->off_offsets = o; o += sizeof(uint32_t) * RS_MAX_PASSES * RS_RADIX;
   l->off_plan = o; o += 256;
@@ -1005,6 +1296,16 @@ int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
   p.tiles = l.tiles;
   p.d_error = ctx->d_error;
 
+  // Short sorts of plain keys go to one cluster.
+  if (p.n <= SS_MAX_N && key_mode == PD_KEY_PLAIN && dbits == RS_RADIX_BITS && !v64 && !offsets_out) {
+    auto k = p.has_vals ? k_sort_cluster<true> : k_sort_cluster<false>;
+    const size_t smem = ss_smem_bytes(p.has_vals != 0);
+    PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned ctas = (unsigned)std::min<uint64_t>(SS_CLUSTER, std::max<uint64_t>(1, pd_ceil_div(p.n, SS_MIN_CHUNK)));
+    pd_launch_scope sc(ctx, PIMDAL_KERNEL_SORT_PASS, s);
+    PD_CHECK_CUDA(pd_launch(k, ctas, SS_THREADS, smem, s, ctas, p));
+    return pd_launch_status(ctx);
+  }
   PD_CHECK_CUDA(cudaMemsetAsync(w, 0, l.memset_bytes, s));
   const unsigned hist_blocks =
       (unsigned)std::min<uint64_t>(pd_ceil_div(p.n, (uint64_t)RS_THREADS * 16), (uint64_t)ctx->sm_count * 4);
@@ -1012,20 +1313,18 @@ int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_SORT_HIST, s);
     auto hk = key_mode == PD_KEY_HASH0 ? k_sort_hist<PD_KEY_HASH0>
               : key_mode == PD_KEY_MULHASH ? k_sort_hist<PD_KEY_MULHASH> : k_sort_hist<PD_KEY_PLAIN>;
-    hk<<<hist_blocks ? hist_blocks : 1, RS_THREADS, 0, s>>>(p);
+    PD_CHECK_CUDA(pd_launch(hk, hist_blocks ? hist_blocks : 1, RS_THREADS, 0, s, 1, p));
   }
-  {
+  // a radix partition, or a sort on a single digit of at most 6 bits
+  const bool part = (dbits <= 6 || (l.npasses == 1 && p.end_bit - p.begin_bit <= 6)) && !p.pairs;
+  if (part || !l.small) {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    k_sort_plan<<<1, RS_THREADS, 0, s>>>(p);
-  }
-  {
-    pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
-    unsigned cb = (unsigned)std::min<uint64_t>(pd_ceil_div(p.n, RS_THREADS), (uint64_t)ctx->sm_count * 8);
-    k_sort_copy<<<cb ? cb : 1, RS_THREADS, 0, s>>>(p);
+    const unsigned cb = (unsigned)std::min<uint64_t>(pd_ceil_div(p.n, RS_THREADS), (uint64_t)ctx->sm_count * 8);
+    PD_CHECK_CUDA(pd_launch(k_sort_copy, cb ? cb : 1, RS_THREADS, 0, s, 1, p));
   }
   // Digits of at most 6 bits over key columns (a radix partition, or a sort
   // on a single small digit): the small-radix pass.
-  if ((dbits <= 6 || (l.npasses == 1 && p.end_bit - p.begin_bit <= 6)) && !p.pairs) {
+  if (part) {
     const int val = v64 ? PV_U64 : p.has_vals ? PV_U32 : PV_NONE;
     for (uint32_t q = 0; q < l.npasses; ++q) {
       pd_launch_scope sc(ctx, PIMDAL_KERNEL_PARTITION, s);
@@ -1034,7 +1333,8 @@ int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
       PartKernel k = pick_part(qbits, val, key_mode);
       const int smem = (int)pp_smem_bytes((int)qbits, val);
       PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      k<<<resident_grid(ctx, (const void *)k, smem, l.tiles), RS_THREADS, smem, s>>>(p, q, shift);
+      PD_CHECK_CUDA(pd_launch(k, resident_grid(ctx, (const void *)k, smem, l.tiles), RS_THREADS, smem, s, 1,
+                              p, q, shift));
     }
     return pd_launch_status(ctx);
   }
@@ -1043,10 +1343,11 @@ int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
     const uint32_t shift = p.begin_bit + q * RS_RADIX_BITS;
     const uint32_t bits = std::min<uint32_t>(RS_RADIX_BITS, p.end_bit - shift);
     const uint32_t mask = (1u << bits) - 1u;
-    auto k = pick_pass(p.has_vals != 0, key_mode);
-    const int smem = (p.has_vals ? 8 : 4) * RS_TILE;
+    auto k = pick_pass(p.has_vals != 0, key_mode, l.small);
+    const int smem = (int)rs_smem_bytes(l.small ? RS_SMALL_ITEMS : RS_ITEMS, p.has_vals != 0);
     PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k<<<resident_grid(ctx, (const void *)k, smem, l.tiles), RS_THREADS, smem, s>>>(p, q, shift, mask);
+    PD_CHECK_CUDA(pd_launch(k, resident_grid(ctx, (const void *)k, smem, l.tiles), RS_THREADS, smem, s, 1,
+                            p, q, shift, mask));
   }
   return pd_launch_status(ctx);
 }

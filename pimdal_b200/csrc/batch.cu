@@ -223,13 +223,14 @@ extern "C" int pimdal_hash_join_batch_create(pimdal_ctx_t *ctx,
   const size_t o_tile0 = c.take(8ull * (count + 1));
   const size_t o_items = c.take(sizeof(uint2) * bitems.size());
   const size_t o_head = c.take(32ull * count);
-  const size_t o_status = c.take(8 * tile0[count]);
+  const size_t status_bytes = 8 * pd_align_up(tile0[count], PD_STATUS_BLOCK);
+  const size_t o_status = c.take(status_bytes);
   const size_t o_tab = c.take(8 * words);
   pimdal_batch *b;
   int st = alloc_plan(ctx, PIMDAL_BATCH_HASH_JOIN, count, c.off, &b);
   if (st) return st;
   char *m = (char *)b->mem;
-  if (cudaMemset(m + o_status, 0, 8 * tile0[count]) != cudaSuccess) {
+  if (cudaMemset(m + o_status, 0, status_bytes) != cudaSuccess) {
     pimdal_batch_destroy(b);
     return PIMDAL_ERR_CUDA;
   }

@@ -70,7 +70,7 @@ struct pd_hj_batch {
   unsigned long long *tables;   // all instances' tables, contiguous
   uint64_t table_words;
   uint32_t *headers;            // 8 words per instance
-  uint64_t *status;             // total_tiles look-back words
+  uint64_t *status;             // total_tiles look-back words, rounded up to a block of them
   uint32_t *epoch;              // device epoch of the look-back words
   uint32_t *counters;           // claim counters (2 words, self-resetting)
   uint32_t *d_error;

@@ -102,6 +102,7 @@ struct JoinParams {
   uint32_t *out_pay, *out_row;
   uint64_t cap;
   uint64_t *status;
+  uint64_t status0;             // first look-back word of the chain
   uint32_t epoch;
   uint32_t *claim;
   uint32_t *d_error;
@@ -220,7 +221,7 @@ __device__ __noinline__ uint32_t emit_all(const unsigned long long *table, uint3
 }
 
 // One probe tile: rows [row0, min(row0 + HJ_TILE, hi)) of p, tile index gtile
-// in p.status (the tile with index 0 starts the chain).  When count_last,
+// of its chain (the tile with index 0 starts it).  When count_last,
 // the tile also stores the inclusive match count in *p.d_count.
 __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0, uint64_t hi,
                                               uint64_t gtile, uint32_t side, bool stop_first,
@@ -337,7 +338,8 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
   }
   if (gtile == 0) {
     if (tid == 0) {
-      pd_store_relaxed_u64(p.status, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, total));
+      pd_store_relaxed_u64(p.status + pd_status_index(p.status0),
+                           pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, total));
       s_prefix = 0;
     }
   } else {
@@ -345,10 +347,12 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
     // below without taking issue slots from the SM's other CTAs.
     if (warp == 0) {
       if (lane == 0)
-        pd_store_relaxed_u64(p.status + gtile, pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
-      const uint64_t pre = pd_lookback_warp(p.status, (int64_t)gtile, p.epoch, p.d_error);
+        pd_store_relaxed_u64(p.status + pd_status_index(p.status0 + gtile),
+                             pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
+      const uint64_t pre = pd_lookback_warp(p.status, (int64_t)gtile, p.epoch, p.d_error, p.status0);
       if (lane == 0) {
-        pd_store_relaxed_u64(p.status + gtile, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, pre + total));
+        pd_store_relaxed_u64(p.status + pd_status_index(p.status0 + gtile),
+                             pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, pre + total));
         s_prefix = pre;
       }
     }
@@ -431,7 +435,7 @@ __global__ void __launch_bounds__(HJ_THREADS, PD_HJ_MIN_CTAS) k_hj_probe(JoinPar
     // the inclusive count this thread has just published (inside the tile's
     // code the count costs registers that it does not have: 1% slower)
     if (tl == tiles - 1 && tid == 0)
-      *p.d_count = pd_load_relaxed_u64(p.status + tl) & PD_STATUS_VALUE_MASK;
+      *p.d_count = pd_load_relaxed_u64(p.status + pd_status_index(tl)) & PD_STATUS_VALUE_MASK;
   }
 }
 
@@ -460,7 +464,8 @@ __device__ __forceinline__ JoinParams hjb_params(const pd_hj_batch &b, const pd_
   p.out_pay = in.out_pay;
   p.out_row = in.out_row;
   p.cap = in.cap;
-  p.status = b.status + in.tile0;
+  p.status = b.status;
+  p.status0 = in.tile0;
   p.d_error = b.d_error;
   p.d_count = in.d_count;
   return p;
@@ -478,7 +483,8 @@ __global__ void k_hjb_begin(pd_hj_batch b) {
 __global__ void __launch_bounds__(256) k_hjb_status_clear(pd_hj_batch b) {
   if (*b.epoch != 1u) return;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b.total_tiles; i += stride)
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < pd_align_up(b.total_tiles, PD_STATUS_BLOCK);
+       i += stride)
     b.status[i] = 0;
 }
 
@@ -802,10 +808,10 @@ __global__ void __launch_bounds__(HJS_THREADS, 1) k_hjs_join(JoinSmemParams p) {
         if (tid == 0) pd_store_relaxed_u64(p.status, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, total));
       } else {
         if (tid == 0)
-          pd_store_relaxed_u64(p.status + q, pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
+          pd_store_relaxed_u64(p.status + pd_status_index(q), pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
         pre = pd_lookback_warp(p.status, (int64_t)q, p.epoch, p.d_error);
         if (tid == 0)
-          pd_store_relaxed_u64(p.status + q, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, pre + total));
+          pd_store_relaxed_u64(p.status + pd_status_index(q), pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, pre + total));
       }
       if (tid == 0) {
         s_prefix = pre;

@@ -152,14 +152,13 @@ __global__ void __launch_bounds__(SEL_THREADS) k_select(SelParams p) {
     const uint32_t total = __shfl_sync(0xffffffffu, xi, 31);
     uint64_t prefix = 0;
     if (tile == 0) {
-      if (lane == 0) pd_store_release_u64(p.status, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, total));
+      if (lane == 0) pd_store_relaxed_u64(p.status, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, total));
     } else {
-      if (lane == 0)
-        pd_store_release_u64(p.status + tile, pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
+      uint64_t *word = p.status + pd_status_index(tile);
+      if (lane == 0) pd_store_relaxed_u64(word, pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
       prefix = pd_lookback_warp(p.status, (int64_t)tile, p.epoch, p.d_error);
       if (lane == 0)
-        pd_store_release_u64(p.status + tile,
-                             pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, prefix + total));
+        pd_store_relaxed_u64(word, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, prefix + total));
     }
     if (lane == 0) {
       s_prefix = prefix;
@@ -299,9 +298,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_select_chunked(SlParams q) {
       const uint32_t slot = consumed % SL_STAGES, parity = (consumed / SL_STAGES) & 1u;
       const uint32_t b = (uint32_t)min((uint64_t)SL_STAGE_BYTES, bulk_bytes - (uint64_t)j * SL_STAGE_BYTES);
       uint32_t spins = 0;
-      const uint64_t t0 = pd_globaltimer_ns();
+      uint64_t t0 = 0;
       while (!pd_mbar_try_wait(&s_bar[slot], parity)) {
-        if (pd_wait_expired(p.d_error, t0, ++spins)) break;
+        if (pd_wait_expired(p.d_error, &t0, ++spins)) break;
       }
       const uint4 *v = reinterpret_cast<const uint4 *>(s_ring + slot * SL_STAGE_BYTES);
       for (uint32_t i = tid; i < b / 16; i += SL_THREADS) {
@@ -461,9 +460,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_select_chunked(SlParams q) {
       const uint32_t uses = (issued - slot + SL_STAGES - 1) / SL_STAGES;  // issues on this slot
       const uint32_t parity = (uses - 1) & 1u;
       uint32_t spins = 0;
-      const uint64_t t0 = pd_globaltimer_ns();
+      uint64_t t0 = 0;
       while (!pd_mbar_try_wait(&s_bar[slot], parity)) {
-        if (pd_wait_expired(p.d_error, t0, ++spins)) break;
+        if (pd_wait_expired(p.d_error, &t0, ++spins)) break;
       }
     }
   }
@@ -546,9 +545,9 @@ __device__ __forceinline__ bool co_grid_barrier(uint32_t *bar, uint32_t *d_error
       pd_store_release_u32(bar + 1, gen + 1);
     } else {
       uint32_t spins = 0;
-      const uint64_t t0 = pd_globaltimer_ns();
+      uint64_t t0 = 0;
       while (pd_load_acquire_u32(bar + 1) == gen) {
-        if (pd_wait_expired(d_error, t0, ++spins)) break;
+        if (pd_wait_expired(d_error, &t0, ++spins)) break;
         __nanosleep(32);
       }
     }

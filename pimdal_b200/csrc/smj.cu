@@ -209,10 +209,10 @@ __global__ void __launch_bounds__(MJ_THREADS, 5) k_smj_merge(MergeParams p) {
     // below without taking issue slots from the SM's other CTAs.
     if (warp == 0) {
       if (lane == 0)
-        pd_store_relaxed_u64(p.status + tile, pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
+        pd_store_relaxed_u64(p.status + pd_status_index(tile), pd_pack_status(p.epoch, PD_FLAG_AGGREGATE, total));
       const uint64_t pre = pd_lookback_warp(p.status, (int64_t)tile, p.epoch, p.d_error);
       if (lane == 0) {
-        pd_store_relaxed_u64(p.status + tile, pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, pre + total));
+        pd_store_relaxed_u64(p.status + pd_status_index(tile), pd_pack_status(p.epoch, PD_FLAG_INCLUSIVE, pre + total));
         s_prefix = pre;
       }
     }

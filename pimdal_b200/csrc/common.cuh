@@ -211,6 +211,17 @@ __device__ __forceinline__ uint64_t pd_load_relaxed_u64(const uint64_t *p) {
   return v;
 }
 
+// Adds v to a 64-bit shared sum held as two words.  Shared memory adds 32-bit
+// words natively but 64-bit ones in a compare-and-swap loop.  The low words'
+// additions wrap exactly once per carry, and the addition that wraps passes
+// its carry on, so the sum is exact mod 2^64 in any order.
+__device__ __forceinline__ void pd_smem_add64(uint32_t *lo, uint32_t *hi, unsigned long long v) {
+  const uint32_t l = (uint32_t)v;
+  const uint32_t old = atomicAdd(lo, l);
+  const uint32_t h = (uint32_t)(v >> 32) + (uint32_t)(old + l < l);
+  if (h) atomicAdd(hi, h);
+}
+
 // ---- TMA bulk copies (non-multicast, this CTA's own shared memory) --------
 __device__ __forceinline__ uint32_t pd_smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);

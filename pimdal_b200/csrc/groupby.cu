@@ -179,17 +179,6 @@ __device__ __forceinline__ uint32_t gb_bucket2(uint32_t x, uint32_t nb) {
   return __umulhi(x * 0xC2B2AE3Du, nb);
 }
 
-// Adds v to a 64-bit shared sum held as two words.  Shared memory adds 32-bit
-// words natively but 64-bit ones in a compare-and-swap loop.  The low words'
-// additions wrap exactly once per carry, and the addition that wraps passes
-// its carry on, so the sum is exact mod 2^64 in any order.
-__device__ __forceinline__ void smem_add64(uint32_t *lo, uint32_t *hi, unsigned long long v) {
-  const uint32_t l = (uint32_t)v;
-  const uint32_t old = atomicAdd(lo, l);
-  const uint32_t h = (uint32_t)(v >> 32) + (uint32_t)(old + l < l);
-  if (h) atomicAdd(hi, h);
-}
-
 __device__ __forceinline__ int bucket_match(const uint4 &q, uint32_t key) {
   return q.x == key ? 0 : q.y == key ? 1 : q.z == key ? 2 : q.w == key ? 3 : -1;
 }
@@ -312,7 +301,7 @@ __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, 
     for (int r = 0; r < 4; ++r) {
       if (slot[r] >= 0) {
         atomicAdd(t.cnt + acc[r], 1u);
-        smem_add64(t.slo + acc[r], t.shi + acc[r], (unsigned long long)v[r]);
+        pd_smem_add64(t.slo + acc[r], t.shi + acc[r], (unsigned long long)v[r]);
       }
     }
 #pragma unroll

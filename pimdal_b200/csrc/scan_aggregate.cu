@@ -17,11 +17,11 @@
 //    materialisation, at sector granularity.
 //  * Sums accumulate in shared memory in nsets copies of the table ([slot]
 //    [set] layout): thread t adds into set t mod nsets, with plain adds when
-//    every thread has its own set (nsets = 256) and shared-memory atomics
-//    otherwise.  The host picks the most sets whose tables fit in
+//    every thread has its own set (nsets = 256) and 32-bit shared-memory
+//    atomics otherwise.  The host picks the most sets whose tables fit in
 //    PD_SA_SMEM_TARGET bytes, so a small key space gets private slots and a
 //    mid-sized one (TPC-H Q1: 6 keys x 6 sums) keeps the CTA small enough for
-//    8 CTAs per SM; a large key space gets one shared table.  Each CTA
+//    7 CTAs per SM; a large key space gets one shared table.  Each CTA
 //    then adds its non-zero slots to a global table with one atomic each, and
 //    one CTA emits the groups with rows, in key order.  Integer sums wrap mod
 //    2^64 and do not depend on the order of the additions.
@@ -35,12 +35,15 @@ constexpr int SA_THREADS = 256;
 #ifndef PD_SA_UNROLL
 #define PD_SA_UNROLL 4  // rows per thread per step
 #endif
+#ifndef PD_SA_CTAS
+#define PD_SA_CTAS 7  // per SM
+#endif
 #ifndef PD_SA_EAGER
 #define PD_SA_EAGER 0   // 1: predicate columns read for every row, not only the selected ones
 #endif
 constexpr int SA_UNROLL = PD_SA_UNROLL;
 #ifndef PD_SA_SMEM_TARGET
-#define PD_SA_SMEM_TARGET (24 * 1024)  // shared-memory bytes of the table copies
+#define PD_SA_SMEM_TARGET (16 * 1024)  // shared-memory bytes of the table copies
 #endif
 
 struct SaCol {
@@ -63,6 +66,7 @@ struct SaParams {
   int64_t tadd[PIMDAL_SA_MAX_EXPRS][PIMDAL_SA_MAX_TERMS];
   uint32_t tneg[PIMDAL_SA_MAX_EXPRS][PIMDAL_SA_MAX_TERMS];
   uint32_t nterms[PIMDAL_SA_MAX_EXPRS];
+  uint32_t tfirst[PIMDAL_SA_MAX_EXPRS];  // first term not in the expression before
   uint32_t nexprs;
   uint32_t nsets;                   // table copies (a power of two, 1 .. SA_THREADS)
   unsigned long long *g_acc;        // [ks][nexprs + 1] (slot 0: COUNT)
@@ -96,10 +100,13 @@ __device__ __forceinline__ void sa_load_rows(const SaCol &c, const uint32_t (&ro
   }
 }
 
-// 5 CTAs per SM (48 registers, a 40-byte spill): the scan is bound by the
-// latency of its dependent column loads, and 5 CTAs hide more of it than 4
-// at 64 registers (Q6 0.50 -> 0.43 ms, Q1 1.12 -> 0.98 ms on 6e7 rows).
-__global__ void __launch_bounds__(SA_THREADS, 5) k_sa_scan(SaParams p) {
+// Bound by instructions and the latency between them: fetching the columns ahead
+// made it slower (Q1 0.91 -> 0.98 ms), fewer terms, cheaper sums and more warps
+// make it faster.  On 6e7 rows, Q1 and Q6: 0.98 and 0.44 ms; with sums of two
+// 32-bit words 0.95 and 0.44; terms shared between expressions 0.85 and 0.43;
+// and 7 CTAs per SM at 32 registers instead of 5 at 48, 0.75 and 0.39 (6 CTAs
+// 0.77 and 0.40, 8 CTAs 0.75 and 0.39).
+__global__ void __launch_bounds__(SA_THREADS, PD_SA_CTAS) k_sa_scan(SaParams p) {
   pd_grid_dep();
   extern __shared__ __align__(16) unsigned long long sa_acc[];
   const int tid = threadIdx.x;
@@ -108,12 +115,16 @@ __global__ void __launch_bounds__(SA_THREADS, 5) k_sa_scan(SaParams p) {
   const uint32_t nsets = p.nsets;
   const uint32_t words = slots * nsets;
   const uint32_t set = tid & (nsets - 1);  // this thread's copy of the table
+  // a copy of its own holds 64-bit words; shared ones are two arrays of 32-bit
+  // words, low then high (pd_smem_add64), and a count needs the low word only
+  uint32_t *lo = reinterpret_cast<uint32_t *>(sa_acc), *hi = lo + words;
   for (uint32_t i = tid; i < words; i += SA_THREADS) sa_acc[i] = 0;
   __syncthreads();
-  auto acc_add = [=](uint32_t key, uint32_t slot, unsigned long long v) {
-    const uint32_t i = (key * nv + slot) * nsets + set;
-    if (nsets == SA_THREADS) sa_acc[i] += v;
-    else atomicAdd(&sa_acc[i], v);
+  // i: the key's first slot in this thread's copy, slot: slot * nsets
+  auto acc_add = [=](uint32_t i, uint32_t slot, unsigned long long v) {
+    if (nsets == SA_THREADS) sa_acc[i + slot] += v;
+    else if (slot == 0) atomicAdd(lo + i, (uint32_t)v);  // fewer than 2^32 rows
+    else pd_smem_add64(lo + i + slot, hi + i + slot, v);
   };
   // one key (no group columns): the sums stay in registers until the end
   const bool scalar = p.ks == 1;
@@ -165,17 +176,19 @@ __global__ void __launch_bounds__(SA_THREADS, 5) k_sa_scan(SaParams p) {
         ok[u] = false;
       }
       if (scalar) racc[0] += ok[u] ? 1ull : 0ull;
-      else if (ok[u]) acc_add(key[u], 0, 1ull);
+      key[u] = key[u] * nv * nsets + set;
+      if (!scalar && ok[u]) acc_add(key[u], 0, 1ull);
     }
+    // An expression that begins with all the terms of the one before (TPC-H
+    // Q1: price, price * (100 - discount), that * (100 + tax)) goes on from its
+    // product; the scan is bound by instructions, and 8 terms become 5 there.
+    unsigned long long val[SA_UNROLL];
 #pragma unroll
     for (int e = 0; e < PIMDAL_SA_MAX_EXPRS; ++e) {
       if (e >= (int)p.nexprs) continue;
-      unsigned long long val[SA_UNROLL];
-#pragma unroll
-      for (int u = 0; u < SA_UNROLL; ++u) val[u] = 1ull;
 #pragma unroll
       for (int t = 0; t < PIMDAL_SA_MAX_TERMS; ++t) {
-        if (t < (int)p.nterms[e]) {
+        if (t >= (int)p.tfirst[e] && t < (int)p.nterms[e]) {
           const SaCol c = p.tc[e][t];
           const uint32_t neg = p.tneg[e][t];
           const int64_t add = p.tadd[e][t];
@@ -187,26 +200,35 @@ __global__ void __launch_bounds__(SA_THREADS, 5) k_sa_scan(SaParams p) {
             for (int u = 0; u < SA_UNROLL; ++u) x[u] = 0;
           }
 #pragma unroll
-          for (int u = 0; u < SA_UNROLL; ++u) val[u] *= (unsigned long long)((neg ? -x[u] : x[u]) + add);
+          for (int u = 0; u < SA_UNROLL; ++u) {
+            const unsigned long long y = (unsigned long long)((neg ? -x[u] : x[u]) + add);
+            val[u] = t ? val[u] * y : y;
+          }
         }
       }
 #pragma unroll
       for (int u = 0; u < SA_UNROLL; ++u) {
         if (scalar) racc[1 + e] += ok[u] ? val[u] : 0ull;
-        else if (ok[u]) acc_add(key[u], 1 + e, val[u]);
+        else if (ok[u]) acc_add(key[u], (1 + e) * nsets, val[u]);
       }
     }
   }
   if (scalar) {
 #pragma unroll
     for (int e = 0; e <= PIMDAL_SA_MAX_EXPRS; ++e)
-      if (e < (int)nv && racc[e]) acc_add(0, e, racc[e]);
+      if (e < (int)nv && racc[e]) {
+        // (a thread's own count may be beyond 32 bits only with its own copy)
+        acc_add(set, e * nsets, racc[e]);
+      }
   }
   if (bad) atomicOr(p.d_error, PD_DEVERR_ARG);
   __syncthreads();
   for (uint32_t s = tid; s < slots; s += SA_THREADS) {
     unsigned long long v = 0;
-    for (uint32_t t = 0; t < nsets; ++t) v += sa_acc[s * nsets + t];
+    for (uint32_t t = 0; t < nsets; ++t) {
+      const uint32_t i = s * nsets + t;
+      v += nsets == SA_THREADS ? sa_acc[i] : (unsigned long long)hi[i] << 32 | lo[i];
+    }
     if (v) atomicAdd(&p.g_acc[s], v);
   }
 }
@@ -371,6 +393,16 @@ extern "C" int pimdal_select_aggregate(pimdal_ctx_t *ctx,
     const pimdal_expr_t &x = a->expr[e];
     if (x.n_terms == 0 || x.n_terms > PIMDAL_SA_MAX_TERMS) return PIMDAL_ERR_ARG;
     p.nterms[e] = x.n_terms;
+    p.tfirst[e] = 0;
+    if (e && a->expr[e - 1].n_terms < x.n_terms) {
+      uint32_t t = 0;
+      for (const pimdal_expr_t &w = a->expr[e - 1]; t < w.n_terms; ++t)
+        if (w.term[t].col != x.term[t].col || w.term[t].add != x.term[t].add ||
+            (x.term[t].col && (w.term[t].dtype != x.term[t].dtype ||
+                               (w.term[t].negate != 0) != (x.term[t].negate != 0))))
+          break;
+      if (t == a->expr[e - 1].n_terms) p.tfirst[e] = t;
+    }
     for (uint32_t t = 0; t < x.n_terms; ++t) {
       const pimdal_term_t &term = x.term[t];
       if (term.col && !sa_dtype_ok(term.dtype)) return PIMDAL_ERR_ARG;

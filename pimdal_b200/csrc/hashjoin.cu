@@ -1389,8 +1389,12 @@ namespace {
 
 constexpr int SJA_THREADS = 256;
 constexpr int SJA_WARPS = SJA_THREADS / 32;
+#ifndef PD_SJA_CTAS
+#define PD_SJA_CTAS 6  // per SM
+#endif
+constexpr int SJA_QUEUE = 31 + 128;      // selected rows of a warp waiting for their chains
 constexpr uint32_t SJA_WARP_KEYS = 256;  // key spaces up to this get one table per warp
-static_assert(PIMDAL_FUSED_MAX_KEYS * 12 <= 48 * 1024, "a CTA-wide table fits 48 KB");
+static_assert(PIMDAL_FUSED_MAX_KEYS * 12 + 4 * SJA_QUEUE * SJA_WARPS <= 227 * 1024, "a CTA-wide table fits");
 static_assert(SJA_WARP_KEYS * SJA_WARPS <= PIMDAL_FUSED_MAX_KEYS, "per-warp tables fit too");
 
 struct SjaParams {
@@ -1411,35 +1415,35 @@ struct SjaParams {
 
 uint32_t sja_tables(uint32_t key_space) { return key_space <= SJA_WARP_KEYS ? SJA_WARPS : 1; }
 
-// 8 CTAs per SM (32 registers): each row's loads and bucket walk form one
-// dependent chain, and twice the warps of the former 4 CTAs per SM hide it
-// (a 6e7-row request 1.03 -> 0.61 ms).
-__global__ void __launch_bounds__(SJA_THREADS, 8) k_sja_aggregate(SjaParams p) {
+// A selected row is one dependent chain: join key, table bucket, columns, sums.
+// Taking each row's chain in the thread that read its date leaves most lanes
+// idle when a query selects a few rows in a hundred, so a warp reads 128 dates
+// (one 16-byte load per lane), appends the selected rows to its queue in
+// shared memory and runs the chains of 32 queued rows at a time (6e7 rows, a
+// quarter selected: 0.59 -> 0.39 ms; 4e6 rows: 50 -> 29 us; 5 or 8 CTAs per SM
+// 0.39 and 0.40 ms).  The sums are two 32-bit words each (pd_smem_add64).
+template <bool VEC>
+__global__ void __launch_bounds__(SJA_THREADS, PD_SJA_CTAS) k_sja_aggregate(SjaParams p) {
   pd_grid_dep();
-  extern __shared__ __align__(16) unsigned long long sja_smem[];
+  extern __shared__ __align__(16) uint32_t sja_smem[];
+  __shared__ uint32_t s_queue[SJA_WARPS][SJA_QUEUE];
   const uint32_t ks = p.key_space;
   const uint32_t tables = ks <= SJA_WARP_KEYS ? SJA_WARPS : 1;
-  unsigned long long *s_sum = sja_smem;                                           // [tables][ks]
-  unsigned int *s_cnt = reinterpret_cast<unsigned int *>(sja_smem + tables * ks);  // [tables][ks]
-  const int tid = threadIdx.x, warp = tid >> 5;
-  for (uint32_t i = tid; i < tables * ks; i += SJA_THREADS) {
-    s_sum[i] = 0;
-    s_cnt[i] = 0;
-  }
+  // [tables][ks]: counts, low and high words of the sums
+  uint32_t *s_cnt = sja_smem, *s_lo = s_cnt + tables * ks, *s_hi = s_lo + tables * ks;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (uint32_t i = tid; i < 3 * tables * ks; i += SJA_THREADS) sja_smem[i] = 0;
   __syncthreads();
-  unsigned long long *my_sum = s_sum + (warp % tables) * ks;
-  unsigned int *my_cnt = s_cnt + (warp % tables) * ks;
+  const uint32_t mine = (warp % tables) * ks;
   const uint32_t gmask = (uint32_t)(((1ull << p.bits) - 1) >> 2);
   const uint32_t side = *p.side_count;
   const bool no_dup = *p.dup_flag == 0;
   bool bad = false;
-  const uint64_t stride = (uint64_t)gridDim.x * SJA_THREADS;
-  for (uint64_t r = (uint64_t)blockIdx.x * SJA_THREADS + tid; r < p.n; r += stride) {
-    const int32_t d = __ldcs(p.date + r);
-    if (d < p.lo || d > p.hi) continue;
+  auto chain = [&](uint32_t r) {
     const uint32_t key = __ldg(p.jkey + r);
     const uint32_t f = p.flag ? __ldg(p.flag + r) : 0u;
-    const int64_t v = __ldg(p.price + r) * (int64_t)(100 - __ldg(p.discount + r));
+    const int64_t price = __ldg(p.price + r);
+    const int32_t discount = __ldg(p.discount + r);
     auto add = [&](uint32_t attr) {
       // the staged glue's key (k_revenue_keys): 32-bit, wrapping
       const uint32_t g = attr * p.attr_mult + f;
@@ -1447,8 +1451,9 @@ __global__ void __launch_bounds__(SJA_THREADS, 8) k_sja_aggregate(SjaParams p) {
         bad = true;
         return;
       }
-      atomicAdd(&my_sum[g], (unsigned long long)v);
-      atomicAdd(&my_cnt[g], 1u);
+      atomicAdd(s_cnt + mine + g, 1u);
+      pd_smem_add64(s_lo + mine + g, s_hi + mine + g,
+                    (unsigned long long)(price * (int64_t)(100 - discount)));
     };
     // the bucket walk of the probe: stop at a bucket with a free slot, or at
     // the first match when the build had no duplicate key
@@ -1473,14 +1478,55 @@ __global__ void __launch_bounds__(SJA_THREADS, 8) k_sja_aggregate(SjaParams p) {
     }
     if (key == 0xFFFFFFFFu)  // build rows equal to the empty word, counted on the side
       for (uint32_t m = 0; m < side; ++m) add(0xFFFFFFFFu);
+  };
+  uint32_t *queue = s_queue[warp];
+  uint32_t queued = 0;  // the same in all lanes
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint64_t stride = (uint64_t)gridDim.x * SJA_WARPS * 128;
+  for (uint64_t r0 = ((uint64_t)blockIdx.x * SJA_WARPS + warp) * 128; r0 < p.n; r0 += stride) {
+    int32_t d[4];
+    uint32_t row[4];
+    bool in[4];
+    if (VEC && r0 + 128 <= p.n) {
+      const int4 v = __ldcs(reinterpret_cast<const int4 *>(p.date + r0) + lane);
+      d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        row[j] = (uint32_t)r0 + 4 * lane + j;
+        in[j] = true;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t r = r0 + 32 * j + lane;
+        row[j] = (uint32_t)r;
+        in[j] = r < p.n;
+        d[j] = in[j] ? __ldcs(p.date + r) : 0;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool sel = in[j] && d[j] >= p.lo && d[j] <= p.hi;
+      const unsigned m = __ballot_sync(0xffffffffu, sel);
+      if (sel) queue[queued + __popc(m & lt)] = row[j];
+      queued += __popc(m);
+    }
+    __syncwarp();
+    while (queued >= 32) {
+      queued -= 32;
+      chain(queue[queued + lane]);
+    }
+    __syncwarp();  // the queue is appended to again
   }
+  if (lane < queued) chain(queue[lane]);
   if (bad) atomicOr(p.d_error, PD_DEVERR_ARG);
   __syncthreads();
   for (uint32_t k = tid; k < ks; k += SJA_THREADS) {
     unsigned long long sum = 0, cnt = 0;
     for (uint32_t t = 0; t < tables; ++t) {
-      sum += s_sum[t * ks + k];
-      cnt += s_cnt[t * ks + k];
+      const uint32_t i = t * ks + k;
+      sum += (unsigned long long)s_hi[i] << 32 | s_lo[i];
+      cnt += s_cnt[i];
     }
     if (cnt) {
       atomicAdd(&p.g_sum[k], sum);
@@ -1578,8 +1624,11 @@ extern "C" int pimdal_select_join_aggregate(pimdal_ctx_t *ctx,
   if (a->size) {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_FUSED, s);
     const size_t smem = 12ull * sja_tables(a->key_space) * a->key_space;
-    const unsigned g = (unsigned)std::min<uint64_t>(pd_ceil_div(a->size, SJA_THREADS), ctx->sm_count * 8ull);
-    PD_CHECK_CUDA(pd_launch(k_sja_aggregate, g, SJA_THREADS, smem, s, 1, p));
+    auto k = ((uintptr_t)a->date & 15u) == 0 ? k_sja_aggregate<true> : k_sja_aggregate<false>;
+    PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned g = (unsigned)std::min<uint64_t>(pd_ceil_div(a->size, 4 * SJA_THREADS),
+                                                    (uint64_t)ctx->sm_count * PD_SJA_CTAS);
+    PD_CHECK_CUDA(pd_launch(k, g, SJA_THREADS, smem, s, 1, p));
   }
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);

@@ -380,13 +380,13 @@ __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, 
   }
 }
 
-__device__ __forceinline__ SmemTable gb_smem_table(unsigned char *smem) {
+__device__ __forceinline__ SmemTable gb_smem_table(unsigned char *smem, uint32_t slots) {
   SmemTable t;
   t.key = reinterpret_cast<uint32_t *>(smem);
-  t.cnt = t.key + GB_SMEM_SLOTS;
-  t.slo = t.cnt + GB_SMEM_SLOTS;
-  t.shi = t.slo + GB_SMEM_SLOTS;
-  t.mm = reinterpret_cast<longlong2 *>(t.shi + GB_SMEM_SLOTS);
+  t.cnt = t.key + slots;
+  t.slo = t.cnt + slots;
+  t.shi = t.slo + slots;
+  t.mm = reinterpret_cast<longlong2 *>(t.shi + slots);
   t.list = nullptr;
   t.nlist = nullptr;
   return t;
@@ -399,8 +399,8 @@ __device__ __forceinline__ void gb_clear_acc(const SmemTable &t, uint32_t i) {
   t.mm[i] = make_longlong2(INT64_MAX, INT64_MIN);
 }
 
-__device__ __forceinline__ void gb_clear_all(const SmemTable &t) {
-  for (uint32_t i = threadIdx.x; i < GB_SMEM_SLOTS; i += GB_THREADS) {
+__device__ __forceinline__ void gb_clear_all(const SmemTable &t, uint32_t slots) {
+  for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) {
     t.key[i] = GB_EMPTY;
     gb_clear_acc(t, i);
   }
@@ -423,7 +423,7 @@ __device__ __forceinline__ void gb_flush(const GbParams &p, const SmemTable &t, 
   const int lane = threadIdx.x & 31;
   const uint32_t n = list ? nl : (mode == GB_LANE ? GB_LANE_SLOTS : GB_SMEM_SLOTS);
   if (mode == GB_LANE) {
-    for (uint32_t i = threadIdx.x >> 5; i < n; i += GB_WARPS) {
+    for (uint32_t i = threadIdx.x >> 5; i < n; i += blockDim.x / 32) {
       const uint32_t j = list ? t.list[i] : i;
       const uint32_t k = t.key[j];
       if (k == GB_EMPTY) continue;
@@ -449,7 +449,7 @@ __device__ __forceinline__ void gb_flush(const GbParams &p, const SmemTable &t, 
   // the CTAs of one launch hold the same groups in about the same slots: each
   // starts elsewhere in its table, so that they do not all update one group
   const uint32_t first = list ? 0u : (uint32_t)((uint64_t)n * blockIdx.x / gridDim.x);
-  for (uint32_t i = threadIdx.x; i < n; i += GB_THREADS) {
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
     const uint32_t j = list ? t.list[i] : (i + first < n ? i + first : i + first - n);
     const uint32_t k = t.key[j];
     if (k == GB_EMPTY) continue;
@@ -467,9 +467,9 @@ __global__ void __launch_bounds__(GB_THREADS, MODE == GB_DIRECT ? 2 : 1)
 k_gb_aggregate(GbParams p, uint32_t pass) {
   pd_grid_trigger();
   extern __shared__ __align__(16) unsigned char gb_smem[];
-  const SmemTable t = gb_smem_table(gb_smem);
+  const SmemTable t = gb_smem_table(gb_smem, GB_SMEM_SLOTS);
   if (MODE != GB_DIRECT) {
-    gb_clear_all(t);
+    gb_clear_all(t, GB_SMEM_SLOTS);
     __syncthreads();
   }
   pd_grid_wait();
@@ -482,18 +482,27 @@ k_gb_aggregate(GbParams p, uint32_t pass) {
   }
 }
 
+// Slots of a chunk's table with CTAS CTAs on an SM.
+constexpr uint32_t gb_chunk_slots(int ctas) { return GB_SMEM_SLOTS / ctas; }
+
 // GB_PART: rows grouped by a hash digit.  Persistent CTAs claim chunks of
 // `chunk` consecutive rows; a chunk goes through the shared table and the
-// slots it claimed are flushed to the global table and reset.
-__global__ void __launch_bounds__(GB_THREADS, 1) k_gb_chunks(GbParams p, uint64_t chunk,
+// slots it claimed are flushed to the global table and reset.  Two CTAs share an
+// SM with half a table each, so that one aggregates while the other claims its
+// chunk's first groups or flushes them (2^22 groups 2.93 -> 2.70 ms, 1e7 rows
+// with 1e5 groups 300 -> 275 us; three with a third 6.9 ms: chunks of two
+// partitions overflow).  gb_layout chooses CTAS.
+template <int CTAS>
+__global__ void __launch_bounds__(GB_THREADS / CTAS, CTAS) k_gb_chunks(GbParams p, uint64_t chunk,
                                                              uint32_t *claim) {
   pd_grid_dep();
+  constexpr uint32_t SLOTS = gb_chunk_slots(CTAS);
   extern __shared__ __align__(16) unsigned char gb_smem[];
   __shared__ uint32_t s_item, s_nlist;
-  SmemTable t = gb_smem_table(gb_smem);
-  t.list = reinterpret_cast<uint16_t *>(gb_smem + GB_SMEM_BYTES);
+  SmemTable t = gb_smem_table(gb_smem, SLOTS);
+  t.list = reinterpret_cast<uint16_t *>(gb_smem + 32ull * SLOTS);
   t.nlist = &s_nlist;
-  gb_clear_all(t);
+  gb_clear_all(t, SLOTS);
   if (threadIdx.x == 0) s_nlist = 0;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = threadIdx.x >> 5;
@@ -512,7 +521,7 @@ __global__ void __launch_bounds__(GB_THREADS, 1) k_gb_chunks(GbParams p, uint64_
     const uint64_t it = s_item;
     if (it >= nchunks) break;
     const uint64_t r0 = it * chunk, r1 = min(r0 + chunk, p.n);
-    gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_WARPS, lane, gb_nbuckets(GB_SMEM));
+    gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_THREADS / CTAS / 32, lane, SLOTS / 4);
     __syncthreads();
     gb_flush(p, t, GB_SMEM, true, s_nlist, true);
     __syncthreads();
@@ -567,10 +576,10 @@ __global__ void __launch_bounds__(256) k_gbb_init(pd_gb_batch b) {
 __global__ void __launch_bounds__(GB_THREADS, 1) k_gbb_aggregate(pd_gb_batch b) {
   extern __shared__ __align__(16) unsigned char gb_smem[];
   __shared__ uint32_t s_item, s_nlist;
-  SmemTable t = gb_smem_table(gb_smem);
+  SmemTable t = gb_smem_table(gb_smem, GB_SMEM_SLOTS);
   t.list = reinterpret_cast<uint16_t *>(gb_smem + GB_SMEM_BYTES);
   t.nlist = &s_nlist;
-  gb_clear_all(t);
+  gb_clear_all(t, GB_SMEM_SLOTS);
   if (threadIdx.x == 0) s_nlist = 0;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = threadIdx.x >> 5;
@@ -1106,6 +1115,7 @@ struct GbLayout {
   int mode;
   uint32_t sub_cap, npasses;
   uint32_t part_bits;   // GB_PART: hash partitions 2^part_bits
+  uint32_t chunk_ctas;  // GB_PART: CTAs per SM that share its shared memory
   size_t gtab, ngroups, ckey, cslot, skey, sslot, sort_ws, pkey, pval, vrange, total;
 };
 
@@ -1171,13 +1181,21 @@ bool gb_layout(const pimdal_aggr_arguments_t *a, GbLayout *l, const GbTune *tune
           : gb_force_direct() ? GB_DIRECT : GB_PART;
   if (tune && tune->mode >= 0 && l->mode >= GB_DIRECT) l->mode = tune->mode;
   l->part_bits = 0;
+  l->chunk_ctas = 2;
   l->pkey = l->pval = 0;
   if (l->mode == GB_PART) {
     uint32_t b = 1;
     while (b < GB_PART_MAX_BITS && (expect >> b) > GB_PART_GROUPS) ++b;
+    // one partition pass fewer, for partitions twice as large (2^28 rows,
+    // 131,072 groups: 6.2 -> 4.3 ms; with 1e7 rows the flushes of the larger
+    // tables cost more than the pass, 0.65 against 0.67 ms)
+    if (b == PD_PART_DIGIT_BITS + 1 && a->size >= (1u << 25)) --b;
     if (tune && tune->mode == GB_PART && tune->part_bits >= 1 && tune->part_bits <= GB_PART_MAX_BITS)
       b = tune->part_bits;
     l->part_bits = b;
+    // a chunk may span two partitions: half an SM's table holds twice
+    // GB_PART_GROUPS (load 3/5), larger partitions take a whole one
+    l->chunk_ctas = (expect >> b) > GB_PART_GROUPS ? 1 : 2;
   }
   // load factor 1/2 for the small tables, 3/4 for the large ones
   uint64_t slots = l->mode >= GB_DIRECT ? expect + expect / 3 + 1 : 2 * expect;
@@ -1513,11 +1531,14 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
     const uint64_t per_sm = pd_ceil_div(a->size, 8ull * ctx->sm_count);
     const uint64_t chunk = std::max<uint64_t>(
         4096, pd_align_up(std::min<uint64_t>(a->size >> l.part_bits, per_sm), 1024));
-    const unsigned grid = (unsigned)std::min<uint64_t>(pd_ceil_div(a->size, chunk), ctx->sm_count);
-    const size_t smem = pd_gb_batch_shared_bytes();
+    const unsigned grid = (unsigned)std::max<uint64_t>(
+        1, std::min<uint64_t>(pd_ceil_div(a->size, chunk), (uint64_t)l.chunk_ctas * ctx->sm_count));
+    auto k = l.chunk_ctas == 2 ? k_gb_chunks<2> : k_gb_chunks<1>;
+    const size_t smem = 34ull * gb_chunk_slots((int)l.chunk_ctas);
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_GROUP, s);
-    PD_CHECK_CUDA(cudaFuncSetAttribute(k_gb_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PD_CHECK_CUDA(pd_launch(k_gb_chunks, grid ? grid : 1, GB_THREADS, smem, s, 1, p, chunk, ctx->d_counters + PD_COUNTER_GROUP));
+    PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PD_CHECK_CUDA(pd_launch(k, grid, GB_THREADS / l.chunk_ctas, smem, s, 1, p, chunk,
+                            ctx->d_counters + PD_COUNTER_GROUP));
   } else if (l.mode == GB_DIRECT) {
     const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count * 2);
     for (uint32_t q = 0; q < l.npasses; ++q) {

@@ -1237,7 +1237,11 @@ int pd_partition(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
                  cudaStream_t s, const uint64_t *in_v64, uint64_t *out_v64) {
   if (a->layout != PIMDAL_LAYOUT_COLUMNS || (in_v64 == nullptr) != (out_v64 == nullptr))
     return PIMDAL_ERR_ARG;
-  return pd_sort_core(ctx, a, key_mode, ws, s, nullptr, nullptr, PD_PART_DIGIT_BITS, in_v64, out_v64);
+  // as few passes as possible, of about the same width
+  const uint32_t bits = (a->end_bit ? a->end_bit : 32) - a->begin_bit;
+  const uint32_t passes = std::max(1u, (bits + PD_PART_DIGIT_BITS - 1) / PD_PART_DIGIT_BITS);
+  const uint32_t dbits = (bits + passes - 1) / passes;
+  return pd_sort_core(ctx, a, key_mode, ws, s, nullptr, nullptr, dbits, in_v64, out_v64);
 }
 
 namespace {

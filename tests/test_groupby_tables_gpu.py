@@ -38,3 +38,20 @@ def test_table_modes_and_carries(ctx, groups, expected, offset):
     exp = oracle.group_by(k[offset:], v[offset:])
     for name, want in zip(("key", "sum", "count", "min", "max"), exp):
         assert np.array_equal(outs[name][:g].cpu().numpy(), want), name
+
+
+@pytest.mark.parametrize("groups", [65536, 65537, 100_000, 131_072, 131_073, 300_000])
+def test_partition_counts(ctx, groups):
+    """Around the group count where one partition pass becomes two, and the
+    chunk tables that go with it."""
+    n = 1_500_001
+    rng = np.random.default_rng(groups)
+    keys = rng.permutation(2**22)[:groups].astype(np.int32) * 977
+    k = keys[rng.integers(0, groups, n)]
+    v = rng.integers(-2**40, 2**40, n)
+    res, outs = ops.group_kernel(ctx, torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda(),
+                                 method=L.GROUP_HASH, expected_groups=groups, capacity=groups)
+    ctx.sync()
+    g = int(res.item())
+    for name, want in zip(("key", "sum", "count", "min", "max"), oracle.group_by(k, v)):
+        assert np.array_equal(outs[name][:g].cpu().numpy(), want), name

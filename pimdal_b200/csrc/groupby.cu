@@ -123,8 +123,7 @@ __device__ void global_add_from(const GbParams &p, uint32_t key, uint32_t pass, 
   for (uint32_t t = 0; t < cap; ++t) {
     unsigned long long *slot = base + (uint64_t)s * 4;
     if (!loaded) {
-      a = __ldcg(reinterpret_cast<const ulonglong2 *>(slot));
-      b = __ldcg(reinterpret_cast<const ulonglong2 *>(slot) + 1);
+      pd_load_sector_cg(slot, &a, &b);
     }
     loaded = false;
     unsigned long long w = a.x;
@@ -744,7 +743,8 @@ __global__ void __launch_bounds__(256) k_gb_gather(GatherParams g) {
   const ulonglong2 *t = reinterpret_cast<const ulonglong2 *>(g.gtab);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < lim; i += stride) {
     const uint64_t s = g.sslot[i];
-    const ulonglong2 a = t[2 * s], b = t[2 * s + 1];
+    ulonglong2 a, b;
+    pd_load_sector(t + 2 * s, &a, &b);
     if (g.out_key) g.out_key[i] = g.skey[i];
     if (g.out_sum) g.out_sum[i] = (int64_t)a.y;
     if (g.out_count) g.out_count[i] = (int64_t)(a.x >> 32);

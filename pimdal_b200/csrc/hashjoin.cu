@@ -284,9 +284,7 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
 #pragma unroll
       for (int i = 0; i < HJ_BATCH; ++i) {
         if (active[i]) {
-          const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p.table + 4 * (uint64_t)g[i]);
-          glo[i] = q[0];
-          ghi[i] = q[1];
+          pd_load_sector(p.table + 4 * (uint64_t)g[i], &glo[i], &ghi[i]);
           any = true;
         }
       }
@@ -1460,8 +1458,8 @@ __global__ void __launch_bounds__(SJA_THREADS, PD_SJA_CTAS) k_sja_aggregate(SjaP
     const bool stop_first = no_dup && key != 0xFFFFFFFFu;
     uint32_t b = bucket_of(key, 0, p.bits);
     for (uint64_t step = 0; step <= gmask; ++step) {
-      const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p.table + 4 * (uint64_t)b);
-      const ulonglong2 lo = q[0], hi = q[1];
+      ulonglong2 lo, hi;
+      pd_load_sector(p.table + 4 * (uint64_t)b, &lo, &hi);
       const unsigned long long e[4] = {lo.x, lo.y, hi.x, hi.y};
       bool empty = false, found = false;
 #pragma unroll

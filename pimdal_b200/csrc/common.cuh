@@ -567,9 +567,9 @@ bool pd_pred_interval(const pimdal_pred_t &pr, int64_t *lo, int64_t *hi, uint32_
 int pd_sort_with_workspace(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, void *ws,
                            cudaStream_t s);
 int pd_sort_ex(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode, void *ws,
-               cudaStream_t s, uint32_t **offsets_out);
+               cudaStream_t s);
 int pd_sort_ex2(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode, void *ws,
-                cudaStream_t s, uint32_t **offsets_out, const uint64_t *n_dev);
+                cudaStream_t s, const uint64_t *n_dev);
 // Stable radix partition of key columns by bits [a->begin_bit, a->end_bit) of
 // a key transform, in passes of at most PD_PART_DIGIT_BITS bits, carrying the
 // 32-bit column a->in_ptr -> a->out_ptr (row ids when a->in_ptr is NULL and

@@ -1262,7 +1262,7 @@ int pd_gb_batch_run(pimdal_ctx *ctx, const pd_gb_batch &b, cudaStream_t s) {
   sa.in_ptr = b.cslot;
   sa.out = b.skey;
   sa.out_ptr = b.sslot;
-  if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, b.sort_ws, s, nullptr, (const uint64_t *)b.ngroups)))
+  if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, b.sort_ws, s, (const uint64_t *)b.ngroups)))
     return st;
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
@@ -1274,7 +1274,7 @@ int pd_gb_batch_run(pimdal_ctx *ctx, const pd_gb_batch &b, cudaStream_t s) {
   sa.out_ptr = b.cslot;
   sa.begin_bit = 0;
   sa.end_bit = b.inst_bits;
-  if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, b.sort_ws, s, nullptr, (const uint64_t *)b.ngroups)))
+  if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, b.sort_ws, s, (const uint64_t *)b.ngroups)))
     return st;
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_OTHER, s);
@@ -1487,7 +1487,7 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
     q.n_dev = n_pay;
     if ((st = reduce(q))) return st;
     // row-id path: values gathered by row id
-    if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, ws + l.sort_ws, s, nullptr, n_idx))) return st;
+    if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, ws + l.sort_ws, s, n_idx))) return st;
     q = p;
     q.val = a->in_val;
     q.n_dev = n_idx;
@@ -1561,7 +1561,7 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
   sa.in_ptr = p.cslot;
   sa.out = ws + l.skey;
   sa.out_ptr = (uint32_t *)(ws + l.sslot);
-  if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, ws + l.sort_ws, s, nullptr,
+  if ((st = pd_sort_ex2(ctx, &sa, PD_KEY_PLAIN, ws + l.sort_ws, s,
                         (const uint64_t *)p.ngroups)))
     return st;
   GatherParams g{};

@@ -16,11 +16,11 @@
 //  * Tables are arrays of 64-bit slots (payload << 32 | key) filled with
 //    atomicCAS linear probing.  The one row whose slot word would equal the
 //    empty word (key and payload all ones) is counted on the side.
-//  * A table that fits the L2 budget is built and probed directly.  A larger
-//    one is split by the top bits of a multiplicative hash: both relations
-//    are partitioned, and partition by partition one table buffer (reused, so
-//    it stays L2-resident and is never written back) is cleared, built and
-//    probed.  All partition bounds live on the device; no host sync.
+//  * A table that fits the L2 budget is built and probed directly.  For a
+//    larger one both relations are partitioned by the top bits of the hash
+//    whose top bits are also a key's home bucket, so that the rows of one
+//    partition touch one L2-sized slice of the one table; no partition bounds
+//    are needed, on the device or on the host.
 //  * Bucketized linear probing: a key hashes to a bucket of 4 slots (one
 //    32-byte sector) and takes the first free slot of the first bucket, from
 //    there on, that has one; a lookup reads one sector and is done when the
@@ -29,9 +29,8 @@
 //    thread walks 2 rows at a time in lockstep (their bucket loads in flight
 //    together); match counts are scanned and the tile's output
 //    offset resolved by a decoupled look-back (one warp polls while the rest
-//    of the CTA waits at a barrier) that chains across the per-partition
-//    launches, so the output is in probe order within each
-//    partition, partitions in order.
+//    of the CTA waits at a barrier) , so the output is in
+//    probe order within each partition, partitions in order.
 #include <algorithm>
 
 #include "batch.cuh"
@@ -43,8 +42,8 @@ constexpr int HJ_THREADS = 256;
 #ifndef PD_HJ_ITEMS
 // probe rows per thread of a tile (at most 16: 4 count bits each in 64); 12
 // rows at 4 CTAs per SM (64 registers, a 20-byte spill) measured 3.5% faster
-// than 16 rows at 3 CTAs (the probe of 2^28 rows: 3.08 -> 2.97 ms); 8 rows
-// at 4 or 5 CTAs were slower
+// than 16 rows at 3 CTAs (the probe of 2^28 rows: 3.08 -> 2.97 ms); with
+// buckets read in one load, 2.82 ms against 2.89 with 8 rows at 5 CTAs
 #define PD_HJ_ITEMS 12
 #endif
 constexpr int HJ_ITEMS = PD_HJ_ITEMS;
@@ -76,20 +75,19 @@ uint32_t pd_hj_table_bits(uint64_t nb, uint32_t load_pct) {
 namespace {
 
 // Home bucket of a key: buckets are aligned groups of 4 slots (one 32-byte
-// sector); a table of 2^bits slots has 2^(bits-2) buckets.  The bucket is
-// bits [64 - part_bits - (bits-2), 64 - part_bits) of key * PD_GOLDEN64,
-// just below the bits that chose the partition.  part_bits + bits - 2 <= 30
-// (the table layout caps all partitions together at 2^32 slots), so they all
-// lie in the product's high word, computed here in 32-bit arithmetic.
-__device__ __forceinline__ uint32_t bucket_of(uint32_t key, uint32_t part_bits, uint32_t bits) {
+// sector); a table of 2^bits slots has 2^(bits-2) buckets.  The bucket is the
+// top bits - 2 bits of key * PD_GOLDEN64 (a partitioned join's partition is the
+// topmost of them).  bits <= 32, so they lie in the product's high word,
+// computed here in 32-bit arithmetic.
+__device__ __forceinline__ uint32_t bucket_of(uint32_t key, uint32_t bits) {
   const uint32_t hi = __umulhi(key, (uint32_t)PD_GOLDEN64) + key * (uint32_t)(PD_GOLDEN64 >> 32);
-  return (hi << part_bits) >> (34 - bits);
+  return hi >> (34 - bits);
 }
 
 struct JoinParams {
   // table
   unsigned long long *table;
-  uint32_t bits, part_bits;
+  uint32_t bits;
   uint32_t *side_count;
   uint32_t *dup_flag;           // set by the build when a key occurs twice
   // build side
@@ -135,7 +133,7 @@ __device__ __forceinline__ void hj_insert(const JoinParams &p, uint32_t k, uint3
     return;
   }
   const uint32_t gmask = (uint32_t)(((1ull << p.bits) - 1) >> 2);
-  uint32_t g = bucket_of(k, p.part_bits, p.bits);
+  uint32_t g = bucket_of(k, p.bits);
   bool done = false;
   bool dup = false;
   for (uint64_t t = 0; t <= gmask && !done; ++t) {
@@ -194,11 +192,11 @@ __device__ __forceinline__ bool resolve_bucket(ulonglong2 lo, ulonglong2 hi, uin
 // (The table and output fields are passed by value: a reference to the
 // parameter struct would make every caller copy it to local memory.)
 __device__ __noinline__ uint32_t emit_all(const unsigned long long *table, uint32_t bits,
-                                          uint32_t part_bits, uint32_t *out_pay, uint32_t *out_row,
+                                          uint32_t *out_pay, uint32_t *out_row,
                                           uint64_t cap, uint32_t key, uint64_t w, uint32_t row,
                                           bool *overflow, bool emit) {
   const uint32_t gmask = (uint32_t)(((1ull << bits) - 1) >> 2);
-  uint32_t g = bucket_of(key, part_bits, bits);
+  uint32_t g = bucket_of(key, bits);
   uint32_t c = 0;
   for (uint64_t t = 0; t <= gmask; ++t) {
     bool has_empty = false;
@@ -271,7 +269,7 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
       // from shared memory instead of waiting on a load per row
       rowv[i] = (p.prow && active[i]) ? __ldcs(p.prow + r) : (uint32_t)r;
 #endif
-      g[i] = bucket_of(key[i], p.part_bits, p.bits);
+      g[i] = bucket_of(key[i], p.bits);
       c[i] = 0;
       fk[i] = 0;
     }
@@ -379,7 +377,7 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
       if (c4 == 1) c = 1;
       else if (c4 > 1) {
         bool dummy = false;
-        c = emit_all(p.table, p.bits, p.part_bits, p.out_pay, p.out_row, p.cap, key, 0, 0, &dummy,
+        c = emit_all(p.table, p.bits, p.out_pay, p.out_row, p.cap, key, 0, 0, &dummy,
                      false);  // count only
         if (key == 0xFFFFFFFFu) c += side;
       }
@@ -394,7 +392,7 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
       if (c4 == 1) {
         if (pos < p.cap) { p.out_pay[pos] = s_first[k][tid]; p.out_row[pos] = row; } else overflow = true;
       } else if (c) {
-        uint64_t q = pos + emit_all(p.table, p.bits, p.part_bits, p.out_pay, p.out_row, p.cap, key,
+        uint64_t q = pos + emit_all(p.table, p.bits, p.out_pay, p.out_row, p.cap, key,
                                     pos, row, &overflow, true);
         if (key == 0xFFFFFFFFu) {
           for (uint32_t m2 = 0; m2 < side; ++m2, ++q) {
@@ -450,7 +448,6 @@ __device__ __forceinline__ JoinParams hjb_params(const pd_hj_batch &b, const pd_
   JoinParams p{};
   p.table = in.table;
   p.bits = in.bits;
-  p.part_bits = 0;
   p.side_count = in.header;
   p.dup_flag = in.header + 2;
   p.bkey = in.bkey;
@@ -1113,13 +1110,13 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
     sa.in_ptr = a->build_payload;
     sa.out = ws + l.bk;
     sa.out_ptr = (uint32_t *)(ws + l.bp);
-    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s, nullptr))) return st;
+    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s))) return st;
     sa.nr_elements = a->size_probe;
     sa.in = a->probe_key;
     sa.in_ptr = a->probe_ptr;
     sa.out = ws + l.pk;
     sa.out_ptr = (uint32_t *)(ws + l.pr);
-    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s, nullptr))) return st;
+    if ((st = pd_sort_ex(ctx, &sa, PD_KEY_MULHASH, ws + l.sort_ws, s))) return st;
     p.bkey = (const uint32_t *)(ws + l.bk);
     p.bpay = (const uint32_t *)(ws + l.bp);
     p.pkey = (const uint32_t *)(ws + l.pk);
@@ -1367,7 +1364,7 @@ extern "C" int pimdal_part_kernel(pimdal_ctx_t *ctx, const pimdal_part_arguments
   sa.layout = PIMDAL_LAYOUT_COLUMNS;
   sa.begin_bit = sh;
   sa.end_bit = a->shift;
-  return pd_sort_ex(ctx, &sa, PD_KEY_HASH0, ws, s, nullptr);
+  return pd_sort_ex(ctx, &sa, PD_KEY_HASH0, ws, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1456,7 +1453,7 @@ __global__ void __launch_bounds__(SJA_THREADS, PD_SJA_CTAS) k_sja_aggregate(SjaP
     // the bucket walk of the probe: stop at a bucket with a free slot, or at
     // the first match when the build had no duplicate key
     const bool stop_first = no_dup && key != 0xFFFFFFFFu;
-    uint32_t b = bucket_of(key, 0, p.bits);
+    uint32_t b = bucket_of(key, p.bits);
     for (uint64_t step = 0; step <= gmask; ++step) {
       ulonglong2 lo, hi;
       pd_load_sector(p.table + 4 * (uint64_t)b, &lo, &hi);

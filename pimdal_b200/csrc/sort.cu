@@ -1195,20 +1195,19 @@ extern "C" int pimdal_sort_workspace_size(const pimdal_sort_arguments_t *a, size
 // sort internally, e.g. the sort-merge join and the sort group-by).
 int pd_sort_with_workspace(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, void *ws,
                            cudaStream_t s) {
-  return pd_sort_ex(ctx, a, PD_KEY_PLAIN, ws, s, nullptr);
+  return pd_sort_ex(ctx, a, PD_KEY_PLAIN, ws, s);
 }
 
 // Same, ordering by the digits of a transform of the key (a stable radix
-// partition when the bit range is one digit wide).  *offsets_out, when given,
-// receives the device address of the exclusive digit offsets of pass 0.
+// partition when the bit range is one digit wide).
 int pd_sort_ex(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode, void *ws,
-               cudaStream_t s, uint32_t **offsets_out) {
-  return pd_sort_ex2(ctx, a, key_mode, ws, s, offsets_out, nullptr);
+               cudaStream_t s) {
+  return pd_sort_ex2(ctx, a, key_mode, ws, s, nullptr);
 }
 
 namespace {
 int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode, void *ws,
-                 cudaStream_t s, uint32_t **offsets_out, const uint64_t *n_dev, uint32_t dbits,
+                 cudaStream_t s, const uint64_t *n_dev, uint32_t dbits,
                  const uint64_t *in_v64, uint64_t *out_v64, const int64_t *pay64 = nullptr,
                  const int64_t *pay_min = nullptr);
 }
@@ -1216,8 +1215,8 @@ int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
 // Same, with the element count read on the device from *n_dev (a->nr_elements
 // is then an upper bound that sizes the workspace and the grids).
 int pd_sort_ex2(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode, void *ws,
-                cudaStream_t s, uint32_t **offsets_out, const uint64_t *n_dev) {
-  return pd_sort_core(ctx, a, key_mode, ws, s, offsets_out, n_dev, RS_RADIX_BITS, nullptr, nullptr);
+                cudaStream_t s, const uint64_t *n_dev) {
+  return pd_sort_core(ctx, a, key_mode, ws, s, n_dev, RS_RADIX_BITS, nullptr, nullptr);
 }
 
 // A stable radix partition of key columns by bits [begin_bit, end_bit) of a
@@ -1229,7 +1228,7 @@ size_t pd_partition_workspace(const pimdal_sort_arguments_t *a, bool v64) {
 }
 int pd_sort_pay64(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, void *ws, cudaStream_t s,
                   const uint64_t *n_dev, const int64_t *pay64, const int64_t *pay_min) {
-  return pd_sort_core(ctx, a, PD_KEY_PLAIN, ws, s, nullptr, n_dev, RS_RADIX_BITS, nullptr, nullptr,
+  return pd_sort_core(ctx, a, PD_KEY_PLAIN, ws, s, n_dev, RS_RADIX_BITS, nullptr, nullptr,
                       pay64, pay_min);
 }
 
@@ -1241,7 +1240,7 @@ int pd_partition(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
   const uint32_t bits = (a->end_bit ? a->end_bit : 32) - a->begin_bit;
   const uint32_t passes = std::max(1u, (bits + PD_PART_DIGIT_BITS - 1) / PD_PART_DIGIT_BITS);
   const uint32_t dbits = (bits + passes - 1) / passes;
-  return pd_sort_core(ctx, a, key_mode, ws, s, nullptr, nullptr, dbits, in_v64, out_v64);
+  return pd_sort_core(ctx, a, key_mode, ws, s, nullptr, dbits, in_v64, out_v64);
 }
 
 namespace {
@@ -1258,14 +1257,13 @@ unsigned resident_grid(const pimdal_ctx *ctx, const void *kernel, int smem, uint
 }
 
 int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode, void *ws,
-                 cudaStream_t s, uint32_t **offsets_out, const uint64_t *n_dev, uint32_t dbits,
+                 cudaStream_t s, const uint64_t *n_dev, uint32_t dbits,
                  const uint64_t *in_v64, uint64_t *out_v64, const int64_t *pay64,
                  const int64_t *pay_min) {
   SortLayout l;
   const bool v64 = out_v64 != nullptr;
   if (!sort_layout(a, &l, dbits, v64)) return PIMDAL_ERR_ARG;
   if (v64 && dbits > 6) return PIMDAL_ERR_ARG;  // only the small-radix pass carries them
-  if (offsets_out) *offsets_out = (uint32_t *)((char *)ws + l.off_offsets);
   if (a->nr_elements > RS_COUNT_MASK) return PIMDAL_ERR_ARG;  // < 2^30 elements
   char *w = (char *)ws;
   SortParams p{};
@@ -1301,7 +1299,7 @@ int pd_sort_core(pimdal_ctx *ctx, const pimdal_sort_arguments_t *a, int key_mode
   p.d_error = ctx->d_error;
 
   // Short sorts of plain keys go to one cluster.
-  if (p.n <= SS_MAX_N && key_mode == PD_KEY_PLAIN && dbits == RS_RADIX_BITS && !v64 && !offsets_out) {
+  if (p.n <= SS_MAX_N && key_mode == PD_KEY_PLAIN && dbits == RS_RADIX_BITS && !v64) {
     auto k = p.has_vals ? k_sort_cluster<true> : k_sort_cluster<false>;
     const size_t smem = ss_smem_bytes(p.has_vals != 0);
     PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -1389,7 +1389,8 @@ constexpr int SJA_WARPS = SJA_THREADS / 32;
 #endif
 constexpr int SJA_QUEUE = 31 + 128;      // selected rows of a warp waiting for their chains
 constexpr uint32_t SJA_WARP_KEYS = 256;  // key spaces up to this get one table per warp
-static_assert(PIMDAL_FUSED_MAX_KEYS * 12 + 4 * SJA_QUEUE * SJA_WARPS <= 227 * 1024, "a CTA-wide table fits");
+constexpr int SJA_MAX_SMEM = 12 * PIMDAL_FUSED_MAX_KEYS;  // the largest tables of a CTA
+static_assert(SJA_MAX_SMEM + 4 * SJA_QUEUE * SJA_WARPS <= 227 * 1024, "a CTA-wide table fits");
 static_assert(SJA_WARP_KEYS * SJA_WARPS <= PIMDAL_FUSED_MAX_KEYS, "per-warp tables fit too");
 
 struct SjaParams {
@@ -1620,7 +1621,9 @@ extern "C" int pimdal_select_join_aggregate(pimdal_ctx_t *ctx,
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_FUSED, s);
     const size_t smem = 12ull * sja_tables(a->key_space) * a->key_space;
     auto k = ((uintptr_t)a->date & 15u) == 0 ? k_sja_aggregate<true> : k_sja_aggregate<false>;
-    PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit is the process's, not this call's: the same for every call, so
+    // that no thread lowers it between another's setting it and its launch
+    PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SJA_MAX_SMEM));
     const unsigned g = (unsigned)std::min<uint64_t>(pd_ceil_div(a->size, 4 * SJA_THREADS),
                                                     (uint64_t)ctx->sm_count * PD_SJA_CTAS);
     PD_CHECK_CUDA(pd_launch(k, g, SJA_THREADS, smem, s, 1, p));

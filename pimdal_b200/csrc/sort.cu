@@ -906,7 +906,9 @@ k_part_pass(SortParams p, uint32_t pass, uint32_t shift) {
   const uint32_t src = plan->src[pass], dst = plan->dst[pass];
   const bool first = plan->first[pass] != 0;
   const uint32_t flip = p.flip;
-  const uint32_t mask = S::B - 1;
+  // the 2-bit kernel also takes digits of one bit: the key's bits above the
+  // digit are not part of it
+  const uint32_t mask = BITS > 2 ? S::B - 1 : (1u << min(2u, min(p.dbits, p.end_bit - shift))) - 1u;
   auto dig = [&](uint32_t k) { return (sort_xform<KEY_MODE>(k, flip) >> shift) & mask; };
 
   const int tid = threadIdx.x;
@@ -1110,8 +1112,8 @@ PartKernel pick_part_bits(int val, int key_mode) {
   if (val == PV_U32) return pick_part_mode<BITS, PV_U32>(key_mode);
   return pick_part_mode<BITS, PV_NONE>(key_mode);
 }
-// Digits of 1..6 bits (a 1-bit digit uses the 2-bit kernel: its upper
-// digits stay empty).
+// Digits of 1..6 bits (a 1-bit digit uses the 2-bit kernel, which masks it to
+// one bit: its upper digits stay empty).
 PartKernel pick_part(uint32_t bits, int val, int key_mode) {
   switch (bits) {
     case 1: case 2: return pick_part_bits<2>(val, key_mode);

@@ -45,6 +45,9 @@ constexpr int SA_UNROLL = PD_SA_UNROLL;
 #ifndef PD_SA_SMEM_TARGET
 #define PD_SA_SMEM_TARGET (16 * 1024)  // shared-memory bytes of the table copies
 #endif
+// the largest tables of a CTA: copies up to the target, or one of all slots
+constexpr int SA_MAX_TABLE = 8 * PIMDAL_SA_MAX_KEYS * (PIMDAL_SA_MAX_EXPRS + 1);
+constexpr int SA_MAX_SMEM = SA_MAX_TABLE > PD_SA_SMEM_TARGET ? SA_MAX_TABLE : PD_SA_SMEM_TARGET;
 
 struct SaCol {
   const void *p;
@@ -426,8 +429,10 @@ extern "C" int pimdal_select_aggregate(pimdal_ctx_t *ctx,
   while (p.nsets > 1 && slots * p.nsets * 8 > PD_SA_SMEM_TARGET) p.nsets >>= 1;
   const size_t smem = slots * p.nsets * 8;
   if (a->size) {
+    // the limit is the process's, not this call's: the same for every call, so
+    // that no thread lowers it between another's setting it and its launch
     PD_CHECK_CUDA(cudaFuncSetAttribute(k_sa_scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+                                       SA_MAX_SMEM));
     int per_sm = 0;  // CTAs per SM at this shared-memory size
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sa_scan, SA_THREADS, smem) !=
             cudaSuccess || per_sm <= 0)

@@ -73,3 +73,38 @@ def test_join_pass(spaces):
         assert g == have.numel() and torch.equal(outs["key"][:g].long(), have)
         assert torch.equal(outs["count"][:g], cnt[have]) and torch.equal(outs["sum"][:g], sums[have])
         c.close()
+
+
+@pytest.mark.parametrize("spaces", [(1, 1024), (40, 1000)])
+def test_scan(spaces):
+    n = 1000
+    calls, checks, keep = [], [], []
+    for i, ks in enumerate(spaces):
+        c, stream = ops.Context(0), torch.cuda.Stream()
+        key = column(n, 0, ks, torch.int32, i)
+        val = [column(n, -2**40, 2**40, torch.int64, 10 * i + e) for e in range(6)]
+        a = L.SelectAggregateArguments(size=n, n_preds=0, n_group=1, key_space=ks, n_exprs=6)
+        a.group[0] = L.GroupCol(col=key.data_ptr(), dtype=L.I32, mult=1)
+        outs = [torch.zeros(ks, dtype=torch.int64, device="cuda") for _ in range(7)]
+        out_key = torch.zeros(ks, dtype=torch.int32, device="cuda")
+        res = torch.zeros(1, dtype=torch.int64, device="cuda")
+        for e in range(6):
+            a.expr[e] = ops._expr([val[e]])
+            a.out_sum[e] = outs[e].data_ptr()
+        a.out_key, a.out_count, a.out_capacity = out_key.data_ptr(), outs[6].data_ptr(), ks
+        c.reserve(8 * ks * 7)
+        calls.append(lambda c=c, a=a, res=res, s=stream: c.lib.pimdal_select_aggregate(
+            c.handle, C.byref(a), res.data_ptr(), s.cuda_stream))
+        keep.append((key, val, a))
+        want = [torch.zeros(ks, dtype=torch.int64, device="cuda").index_add_(0, key, v) for v in val]
+        checks.append((c, stream, res, out_key, outs, want + [torch.bincount(key, minlength=ks)]))
+    torch.cuda.synchronize()
+    assert run_threads(calls) == []
+    for c, stream, res, out_key, outs, want in checks:
+        c.sync(stream)
+        have = want[6].nonzero().flatten()
+        g = int(res.item())
+        assert g == have.numel() and torch.equal(out_key[:g].long(), have)
+        for got, w in zip(outs, want):
+            assert torch.equal(got[:g], w[have])
+        c.close()

@@ -157,10 +157,15 @@ int pd_launch_status(pimdal_ctx *ctx);
 PD_HD uint64_t pd_align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 PD_HD uint64_t pd_ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 
-#define PD_CHECK_CUDA(expr)                      \
-  do {                                           \
-    cudaError_t e__ = (expr);                    \
-    if (e__ != cudaSuccess) return PIMDAL_ERR_CUDA; \
+// Returns PIMDAL_ERR_CUDA when expr fails.  The runtime also keeps the error for
+// this thread; it is taken from there, or the thread's next call, which asks
+// with pd_launch_status, would report it as its own.
+#define PD_CHECK_CUDA(expr)        \
+  do {                             \
+    if ((expr) != cudaSuccess) {   \
+      cudaGetLastError();          \
+      return PIMDAL_ERR_CUDA;      \
+    }                              \
   } while (0)
 
 // ---------------------------------------------------------------------------

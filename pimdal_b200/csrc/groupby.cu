@@ -18,9 +18,10 @@
 // {count << 32 | key, sum, min, max}: the claiming compare-and-swap carries
 // the first rows' count, and every later update of the group touches the same
 // sector.  Three aggregation modes, chosen from the expected group count:
-//  - GB_LANE (up to 128 groups): the CTA has one shared table of 212 keys and
+//  - GB_LANE (up to 64 groups): the CTA has one shared table of 212 keys and
 //    each key 32 accumulators, one per lane number, interleaved so that a
-//    warp's updates fall in 32 different banks whatever keys its lanes hold;
+//    warp's updates fall in 32 different banks whatever keys its lanes hold
+//    (a CTA that meets more keys than that goes on in GB_SMEM);
 //  - GB_SMEM (up to a few thousand groups): every row updates the CTA's
 //    shared-memory table (6784 slots, 212 KB, one 1024-thread CTA per SM);
 //  - GB_PART (many groups): the rows (key and value) are first radix-
@@ -46,9 +47,12 @@
 // aggregated.  Kernel time over 2^28 rows, before and after: 16 groups 2.03 ->
 // 0.85 ms, 100 groups 4.66 -> 1.16, 1000 groups 2.47 -> 1.36, 4096 groups
 // 3.24 -> 1.44; the chunks of 2^22 groups 3.86 -> 2.93.  The line between the
-// modes at 128 groups: 100 groups take 1.16 ms with lane accumulators, 130
-// groups 1.39 ms in the CTA table.
-// A row whose group finds no shared slot within 16 buckets goes to the global
+// modes at 64 groups: above, one key or more of most sets of keys finds both
+// its buckets in the small table full, and its rows cost a walk each (calls of
+// 2^26 rows, lane accumulators against the CTA table: 64 groups 336 and 377 us,
+// 80 groups 432 and 379, 128 groups 669 and 378; 2^20 rows of 128 groups 41 and
+// 33 us).
+// A GB_SMEM row whose group finds no shared slot within 16 buckets goes to the global
 // table; shared tables are merged into the global table at the end of each
 // CTA.  A global update reads the slot's sector once (two 16-byte loads
 // issued together), claims an empty slot with one compare-and-swap, and adds
@@ -70,7 +74,7 @@ constexpr uint32_t GB_SMEM_SLOTS = 6784;  // 34 B each (with the claim list) fil
 constexpr uint32_t GB_LANE_SLOTS = GB_SMEM_SLOTS / 32;  // 212 keys with 32 accumulators each
 constexpr uint32_t GB_SMEM_PROBES = 16;  // buckets
 constexpr size_t GB_SMEM_BYTES = 32ull * GB_SMEM_SLOTS;      // 212 KB
-constexpr uint64_t GB_LANE_MAX_GROUPS = 128;                 // GB_LANE at or below (load 3/5)
+constexpr uint64_t GB_LANE_MAX_GROUPS = 64;                  // GB_LANE at or below (load 3/10)
 constexpr uint64_t GB_SMEM_MAX_GROUPS = 4608;                // GB_SMEM at or below (load 2/3)
 constexpr uint64_t GB_L2_BUDGET = 1ull << 40;                // one pass unless overridden
 enum { GB_LANE = 0, GB_SMEM = 1, GB_DIRECT = 2, GB_PART = 3 };
@@ -196,8 +200,10 @@ __device__ __forceinline__ int bucket_used(const uint4 &q) {
 // their neighbours (3.3 ms per 2^28 rows, the walks dominating).  Two lanes
 // may claim a key in both of its buckets at once; each then collects a part
 // of the group's rows and the merge into the global table adds them up.
+// (GB_LANE does not walk: a key that finds both buckets full gets no slot.)
 // (The table's fields are passed by value: a reference would make every caller
 // keep the struct in local memory.)
+template <bool LANE>
 __device__ __noinline__ int smem_find(uint32_t *tkey, uint16_t *list, uint32_t *nlist, uint32_t nb,
                                       uint32_t key) {
   const uint32_t x = gb_mix32(key);
@@ -227,6 +233,7 @@ __device__ __noinline__ int smem_find(uint32_t *tkey, uint16_t *list, uint32_t *
       if (hit >= 0) return (int)(4 * b) + hit;
     }
     const int e = bucket_used(q);
+    if (LANE && e == 4) return -1;
     if (e == 4) {  // full without the key: walk on from the second bucket
       if (i == 0) b = b2;
       b = (b + 1 == nb) ? 0 : b + 1;
@@ -244,11 +251,13 @@ __device__ __noinline__ int smem_find(uint32_t *tkey, uint16_t *list, uint32_t *
 
 // Four rows of one lane: (A) bucket lookups with all four loads in flight,
 // the rare claims and full buckets on a slow path; (B) the updates as
-// straight-line predicated shared atomics.
+// straight-line predicated shared atomics.  Returns the rows that GB_LANE has
+// left out, one bit each.
 template <int MODE>
-__device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, uint32_t pass,
+__device__ __forceinline__ uint32_t gb_rows4(const GbParams &p, const SmemTable &t, uint32_t pass,
                                          const uint32_t (&k)[4], const long long (&v)[4],
                                          uint32_t valid, uint32_t nb) {
+  uint32_t left = 0;
   if constexpr (MODE == GB_DIRECT) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -290,7 +299,13 @@ __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, 
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
-      if (slot[r] == -2) slot[r] = smem_find(t.key, t.list, t.nlist, nb, k[r]);
+      if (slot[r] == -2) {
+        slot[r] = smem_find<MODE == GB_LANE>(t.key, t.list, t.nlist, nb, k[r]);
+        if (MODE == GB_LANE && slot[r] < 0) {
+          slot[r] = -3;
+          left |= 1u << r;
+        }
+      }
     // accumulator of a slot: the slot itself, or this lane's of the slot's 32
     uint32_t acc[4];
 #pragma unroll
@@ -315,7 +330,16 @@ __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, 
     for (int r = 0; r < 4; ++r)
       if (slot[r] == -1) global_add(p, k[r], gb_h(k[r]), 0, 1u, v[r], v[r], v[r]);
   }
+  return left;
 }
+
+// Where a warp goes on: its next quad of rows in the aligned part, its next
+// row in the rest, and this lane's rows of that step which are still to do.
+struct GbPos {
+  uint64_t quad, row;
+  uint32_t left;
+};
+
 
 // Rows [r0, r1) of p by `warps` warps (this one is number gw): 128
 // consecutive rows per warp step, 4 per lane (one 16-byte key load and two
@@ -323,8 +347,10 @@ __device__ __forceinline__ void gb_rows4(const GbParams &p, const SmemTable &t, 
 template <int MODE>
 __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, uint32_t pass,
                                          uint64_t r0, uint64_t r1, uint64_t gw, uint64_t warps,
-                                         int lane, uint32_t nb) {
+                                         int lane, uint32_t nb, const GbPos *from = nullptr,
+                                         GbPos *stop = nullptr) {
   uint64_t done = r0;
+  uint32_t todo = from ? from->left : 0xFu;
   if (p.vec && (r0 & 3u) == 0) {
     const uint64_t q1 = r1 / 4;  // quads of rows
     const uint4 *k4 = reinterpret_cast<const uint4 *>(p.key);
@@ -343,7 +369,7 @@ __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, 
     // the shared-table modes load the next step's rows while this step's are
     // aggregated; direct updates run at 32 registers, which have no room for them
     constexpr bool AHEAD = MODE != GB_DIRECT;
-    uint64_t b = r0 / 4 + gw * 32;
+    uint64_t b = from ? from->quad : r0 / 4 + gw * 32;
     if (AHEAD) load(b + lane);
     for (; b < q1; b += warps * 32) {
       const uint64_t q = b + lane;
@@ -358,12 +384,17 @@ __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, 
       }
       const long long vv[4] = {va.x, va.y, vb.x, vb.y};
       if (AHEAD) load(q + warps * 32);
-      gb_rows4<MODE>(p, t, pass, kk, vv, ok ? 0xFu : 0u, nb);
+      const uint32_t left = gb_rows4<MODE>(p, t, pass, kk, vv, ok ? todo : 0u, nb);
+      todo = 0xFu;
+      if (MODE == GB_LANE && __any_sync(0xffffffffu, left)) {
+        *stop = {b, q1 * 4 + gw * 128, left};
+        return;
+      }
     }
     done = q1 * 4;
   }
   // unaligned input or the last rows: lane-striped groups of four rows
-  for (uint64_t b = done + gw * 128; b < r1; b += warps * 128) {
+  for (uint64_t b = from ? from->row : done + gw * 128; b < r1; b += warps * 128) {
     uint32_t kk[4];
     long long vv[4];
     uint32_t valid = 0;
@@ -375,8 +406,14 @@ __device__ __forceinline__ void gb_range(const GbParams &p, const SmemTable &t, 
       kk[r] = in ? p.key[i] : 0u;
       vv[r] = (in && p.val) ? (long long)p.val[i] : 1ll;
     }
-    gb_rows4<MODE>(p, t, pass, kk, vv, valid, nb);
+    const uint32_t left = gb_rows4<MODE>(p, t, pass, kk, vv, valid & todo, nb);
+    todo = 0xFu;
+    if (MODE == GB_LANE && __any_sync(0xffffffffu, left)) {
+      *stop = {r1, b, left};
+      return;
+    }
   }
+  if (MODE == GB_LANE) *stop = {r1, r1, 0u};
 }
 
 __device__ __forceinline__ SmemTable gb_smem_table(unsigned char *smem, uint32_t slots) {
@@ -460,6 +497,30 @@ __device__ __forceinline__ void gb_flush(const GbParams &p, const SmemTable &t, 
   }
 }
 
+// GB_LANE rows of a CTA.  The group count is the caller's estimate; where it was
+// too low, the 212 keys run out, and every row of a group without a slot would
+// cost a walk and a global update (2^26 rows of 300 groups expected to be 64:
+// 6.0 ms against 0.40).  So a warp stops at its first row without a slot, and once
+// all have stopped or ended the CTA merges the lane accumulators and takes the
+// rows left to the CTA table.  Returns the mode the table is left in.
+__device__ __noinline__ void gb_lane_rest(GbParams p, SmemTable t, uint64_t r0, uint64_t r1, uint64_t gw,
+                                          uint64_t warps, GbPos at) {
+  gb_flush(p, t, GB_LANE, t.list != nullptr, t.list ? *t.nlist : 0u, true);
+  __syncthreads();
+  if (t.list && threadIdx.x == 0) *t.nlist = 0;
+  __syncthreads();
+  gb_range<GB_SMEM>(p, t, 0, r0, r1, gw, warps, threadIdx.x & 31, gb_nbuckets(GB_SMEM), &at);
+}
+
+__device__ __forceinline__ int gb_lane_rows(const GbParams &p, const SmemTable &t, uint64_t r0,
+                                            uint64_t r1, uint64_t gw, uint64_t warps, int lane) {
+  GbPos at;
+  gb_range<GB_LANE>(p, t, 0, r0, r1, gw, warps, lane, gb_nbuckets(GB_LANE), nullptr, &at);
+  if (!__syncthreads_or(at.left != 0)) return GB_LANE;
+  gb_lane_rest(p, t, r0, r1, gw, warps, at);
+  return GB_SMEM;
+}
+
 // Persistent CTAs over all rows.
 template <int MODE>
 __global__ void __launch_bounds__(GB_THREADS, MODE == GB_DIRECT ? 2 : 1)
@@ -474,10 +535,12 @@ k_gb_aggregate(GbParams p, uint32_t pass) {
   pd_grid_wait();
   const uint64_t warps = (uint64_t)gridDim.x * GB_WARPS;
   const uint64_t gw = (uint64_t)blockIdx.x * GB_WARPS + (threadIdx.x >> 5);
-  gb_range<MODE>(p, t, pass, 0, p.n, gw, warps, threadIdx.x & 31, gb_nbuckets(MODE));
+  int left = MODE;
+  if constexpr (MODE == GB_LANE) left = gb_lane_rows(p, t, 0, p.n, gw, warps, threadIdx.x & 31);
+  else gb_range<MODE>(p, t, pass, 0, p.n, gw, warps, threadIdx.x & 31, gb_nbuckets(MODE));
   if (MODE != GB_DIRECT) {
     __syncthreads();
-    gb_flush(p, t, MODE, false, 0, false);
+    gb_flush(p, t, left, false, 0, false);
   }
 }
 
@@ -599,9 +662,9 @@ __global__ void __launch_bounds__(GB_THREADS, 1) k_gbb_aggregate(pd_gb_batch b) 
     const pd_gb_inst &in = b.inst[item.x];
     const GbParams p = gbb_params(b, in);
     const uint64_t r0 = item.y, r1 = min((uint64_t)item.y + b.rows_per_item, in.n);
-    const int mode = (int)in.mode;
+    int mode = (int)in.mode;
     const uint32_t nb = gb_nbuckets(mode);
-    if (mode == GB_LANE) gb_range<GB_LANE>(p, t, 0, r0, r1, warp, GB_WARPS, lane, nb);
+    if (mode == GB_LANE) mode = gb_lane_rows(p, t, r0, r1, warp, GB_WARPS, lane);
     else if (mode == GB_SMEM) gb_range<GB_SMEM>(p, t, 0, r0, r1, warp, GB_WARPS, lane, nb);
     else gb_range<GB_DIRECT>(p, t, 0, r0, r1, warp, GB_WARPS, lane, nb);
     if (mode != GB_DIRECT) {

@@ -38,6 +38,9 @@ constexpr int SA_THREADS = 256;
 #ifndef PD_SA_CTAS
 #define PD_SA_CTAS 7  // per SM
 #endif
+#ifndef PD_SA_LIST_CTAS
+#define PD_SA_LIST_CTAS 5  // per SM, for scans of a row list
+#endif
 #ifndef PD_SA_EAGER
 #define PD_SA_EAGER 0   // 1: predicate columns read for every row, not only the selected ones
 #endif
@@ -108,8 +111,15 @@ __device__ __forceinline__ void sa_load_rows(const SaCol &c, const uint32_t (&ro
 // make it faster.  On 6e7 rows, Q1 and Q6: 0.98 and 0.44 ms; with sums of two
 // 32-bit words 0.95 and 0.44; terms shared between expressions 0.85 and 0.43;
 // and 7 CTAs per SM at 32 registers instead of 5 at 48, 0.75 and 0.39 (6 CTAs
-// 0.77 and 0.40, 8 CTAs 0.75 and 0.39).
-__global__ void __launch_bounds__(SA_THREADS, PD_SA_CTAS) k_sa_scan(SaParams p) {
+// 0.77 and 0.40, 8 CTAs 0.75 and 0.39).  A scan of a row list gathers its
+// columns: 5 CTAs per SM keep enough of them in flight, and 7, which spill what
+// the addresses take, only slow it down (1e7 ascending rows of 3.3e7, one sum 54
+// against 65 us and three 137 against 178; 3.3e7 random rows, three sums by 6
+// keys 3.72 against 3.97 ms and by 1000 keys 3.54 against 5.68).  (The two differ
+// in nothing else: without the list's branch the scan of all rows was compiled
+// to 10% slower code.)
+template <int CTAS>
+__global__ void __launch_bounds__(SA_THREADS, CTAS) k_sa_scan(SaParams p) {
   pd_grid_dep();
   extern __shared__ __align__(16) unsigned long long sa_acc[];
   const int tid = threadIdx.x;
@@ -431,17 +441,17 @@ extern "C" int pimdal_select_aggregate(pimdal_ctx_t *ctx,
   if (a->size) {
     // the limit is the process's, not this call's: the same for every call, so
     // that no thread lowers it between another's setting it and its launch
-    PD_CHECK_CUDA(cudaFuncSetAttribute(k_sa_scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       SA_MAX_SMEM));
+    auto k = a->rows ? k_sa_scan<PD_SA_LIST_CTAS> : k_sa_scan<PD_SA_CTAS>;
+    PD_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SA_MAX_SMEM));
     int per_sm = 0;  // CTAs per SM at this shared-memory size
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sa_scan, SA_THREADS, smem) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, SA_THREADS, smem) !=
             cudaSuccess || per_sm <= 0)
       per_sm = 1;
     const uint64_t want = pd_ceil_div(a->size, (uint64_t)SA_THREADS * SA_UNROLL);
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>(want, (uint64_t)per_sm * ctx->sm_count));
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_SCAN_AGG, s);
-    PD_CHECK_CUDA(pd_launch(k_sa_scan, grid, SA_THREADS, smem, s, 1, p));
+    PD_CHECK_CUDA(pd_launch(k, grid, SA_THREADS, smem, s, 1, p));
   }
   SaOut o{};
   o.key = a->out_key;

@@ -182,14 +182,6 @@ __device__ __forceinline__ void pd_grid_dep() {
   pd_grid_trigger();
   pd_grid_wait();
 }
-__device__ __forceinline__ void pd_store_release_u64(uint64_t *p, uint64_t v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint64_t pd_load_acquire_u64(const uint64_t *p) {
-  uint64_t v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ void pd_store_release_u32(uint32_t *p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }

@@ -26,8 +26,8 @@
 //    shared-memory table (6784 slots, 212 KB, one 1024-thread CTA per SM);
 //  - GB_PART (many groups): the rows (key and value) are first radix-
 //    partitioned by the top bits of a multiplicative hash of the key, in
-//    stable passes of at most 6 bits, into 2^b partitions of about 1024
-//    groups each.  Persistent CTAs then take chunks of consecutive rows (a
+//    stable passes of at most 6 bits, into 2^b partitions of up to 1024
+//    groups each (up to 2048 where that saves a pass).  Persistent CTAs then take chunks of consecutive rows (a
 //    chunk spans one or two partitions), aggregate each chunk in the
 //    shared-memory table and flush the slots it claimed into the global
 //    table -- about one global merge per group instead of global atomics
@@ -54,8 +54,7 @@
 // 33 us).
 // A GB_SMEM row whose group finds no shared slot within 16 buckets goes to the global
 // table; shared tables are merged into the global table at the end of each
-// CTA.  A global update reads the slot's sector once (two 16-byte loads
-// issued together), claims an empty slot with one compare-and-swap, and adds
+// CTA.  A global update reads the slot's sector once (one 32-byte load), claims an empty slot with one compare-and-swap, and adds
 // the count and sum with fire-and-forget reductions; min/max reductions are
 // issued only when the loaded value shows they change the slot.
 // The occupied global slots are then compacted, sorted by key with K-SORT
@@ -78,7 +77,7 @@ constexpr uint64_t GB_LANE_MAX_GROUPS = 64;                  // GB_LANE at or be
 constexpr uint64_t GB_SMEM_MAX_GROUPS = 4608;                // GB_SMEM at or below (load 2/3)
 constexpr uint64_t GB_L2_BUDGET = 1ull << 40;                // one pass unless overridden
 enum { GB_LANE = 0, GB_SMEM = 1, GB_DIRECT = 2, GB_PART = 3 };
-constexpr uint64_t GB_PART_GROUPS = 1024;   // groups per hash partition
+constexpr uint64_t GB_PART_GROUPS = 1024;   // groups per hash partition (twice that with one pass fewer)
 constexpr uint32_t GB_PART_MAX_BITS = 12;
 
 struct GbParams {
@@ -172,6 +171,7 @@ struct SmemTable {
 // multiplicative hash that partitions the rows, so that the keys of one
 // partition spread over the whole table, and cheaper than the 64-bit mix of
 // the global table's slots.  A key has two buckets, both cut from this hash.
+// (The multipliers are 32-bit primes of xxHash, Y. Collet, 2012.)
 __device__ __forceinline__ uint32_t gb_mix32(uint32_t key) {
   uint32_t x = (key ^ (key >> 16)) * 0x9E3779B1u;
   x = (x ^ (x >> 15)) * 0x85EBCA77u;
@@ -1588,8 +1588,9 @@ int group_kernel_tuned(pimdal_ctx_t *ctx, const pimdal_aggr_arguments_t *a,
     p.key = (const uint32_t *)(ws + l.pkey);
     p.val = pval;
     p.vec = 1;
-    // a chunk holds at most about one partition's rows, so at most about
-    // 2 * GB_PART_GROUPS groups; with few partitions it is cut further so
+    // a chunk holds at most about one partition's rows, so at most the groups
+    // of two: about 2 * GB_PART_GROUPS, or twice that in the whole-SM tables
+    // of larger partitions; with few partitions it is cut further so
     // that every SM gets several chunks
     const uint64_t per_sm = pd_ceil_div(a->size, 8ull * ctx->sm_count);
     const uint64_t chunk = std::max<uint64_t>(

@@ -29,8 +29,8 @@
 //    thread walks 2 rows at a time in lockstep (their bucket loads in flight
 //    together); match counts are scanned and the tile's output
 //    offset resolved by a decoupled look-back (one warp polls while the rest
-//    of the CTA waits at a barrier) , so the output is in
-//    probe order within each partition, partitions in order.
+//    of the CTA waits at a barrier), so the output is in probe order within
+//    each partition, partitions in order.
 #include <algorithm>
 
 #include "batch.cuh"

@@ -111,7 +111,9 @@ __device__ __forceinline__ void sa_load_rows(const SaCol &c, const uint32_t (&ro
 // make it faster.  On 6e7 rows, Q1 and Q6: 0.98 and 0.44 ms; with sums of two
 // 32-bit words 0.95 and 0.44; terms shared between expressions 0.85 and 0.43;
 // and 7 CTAs per SM at 32 registers instead of 5 at 48, 0.75 and 0.39 (6 CTAs
-// 0.77 and 0.40, 8 CTAs 0.75 and 0.39).  A scan of a row list gathers its
+// 0.77 and 0.40, 8 CTAs 0.75 and 0.39), although at 32 registers a thread spills
+// (80 bytes of stack, 156 bytes of stores and 412 of loads; the 21 MB of the
+// stacks are what a profile shows as DRAM writes).  A scan of a row list gathers its
 // columns: 5 CTAs per SM keep enough of them in flight, and 7, which spill what
 // the addresses take, only slow it down (1e7 ascending rows of 3.3e7, one sum 54
 // against 65 us and three 137 against 178; 3.3e7 random rows, three sums by 6

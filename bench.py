@@ -50,15 +50,15 @@ NCU_TRAFFIC = {
                     "profiles/k_sort_pass_2p25_pairs.md"),
     "k_select_coop": ((537.0e6 + 39.6e6) / 2**26, "row",
                       "profiles/k_select_coop_2p26.md (2^26 rows; at 2^24 the second read hits L2)"),
-    "k_hj_probe": ((339.5e6 + 90.9e6) / 2**25, "partitioned probe row",
+    "k_hj_probe": ((343.6e6 + 98.7e6) / 2**25, "partitioned probe row",
                    "profiles/k_hj_probe_2p25_probe.md"),
-    "k_gb_aggregate_shared": ((403.1e6 + 5.9e6) / 2**25, "row",
+    "k_gb_aggregate_shared": ((402.9e6 + 3.5e6) / 2**25, "row",
                               "profiles/k_gb_aggregate_2p25_rows.md (4096 groups)"),
     "k_gb_aggregate_direct": ((3528.9e6 + 874.8e6) / 2**25, "row",
                               "profiles/k_gb_aggregate_2p25_rows.md (2^22 groups)"),
-    "k_smj_merge": ((336.1e6 + 215.0e6) / 2**25, "outer row",
+    "k_smj_merge": ((336.0e6 + 217.2e6) / 2**25, "outer row",
                     "profiles/k_smj_merge_2p25_outer.md"),
-    "k_gb_chunks": ((424.5e6 + 7.8e6) / 2**25, "row",
+    "k_gb_chunks": ((424.5e6 + 6.1e6) / 2**25, "row",
                     "profiles/k_gb_chunks_2p25_rows.md (chunk aggregation after partitioning)"),
 }
 

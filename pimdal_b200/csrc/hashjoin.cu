@@ -1130,10 +1130,12 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
   const unsigned clear_grid = (unsigned)std::min<uint64_t>(pd_ceil_div(1ull << l.bits, 512), ctx->sm_count * 8ull);
   const unsigned build_grid = ctx->sm_count * 8;
   const int pgrid = probe_grid(ctx);
-  // Early launches pay where launches count (1e6 probe rows: 37.8 -> 34.3 us);
-  // in a large join the next kernel's waiting CTAs cost more than its launch
-  // (2^28 probe rows, 2^25 build rows: 6.00 -> 6.11 ms).
-  const bool early = a->size_probe < (1u << 24);
+  // Early launches pay where launches count (us with and without: 1e6 probe rows
+  // 32.9 and 36.6, 2^24 rows 235 and 245, 2^25 rows 761 and 767; 2^26 rows the
+  // same); in a larger join the next kernel's waiting CTAs cost more than its
+  // launch (2^28 rows 5.69 and 5.54 ms).  A build or a probe by itself and the
+  // partition passes lose nothing at any size and are always launched early.
+  const bool early = a->size_probe < (1u << 26);
   // One table of 2^bits slots, one build and one probe launch over the
   // (partitioned) rows.  A key's home bucket is the top bits of the same hash
   // whose top part_bits chose its partition, so the rows of partition q touch

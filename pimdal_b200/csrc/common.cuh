@@ -212,14 +212,21 @@ __device__ __forceinline__ uint64_t pd_load_relaxed_u64(const uint64_t *p) {
 // at random spend a tag lookup in L1 per lane and instruction, so two 16-byte
 // loads cost twice as much (join probe of 2^28 rows 3.00 -> 2.82 ms; flushes of
 // the chunks of 2^22 groups 2.69 -> 2.36 ms; no gain in the join's build, which
-// waits for its compare-and-swap).  The line gets a place in L1: without one
-// (2.77 ms) the reads of a small table, or of the hot keys of a skewed probe,
-// all go to the same few lines of L2 (2^26 rows against 100 build rows 2.23
-// instead of 0.54 ms; against 10^6 with half of the rows on 20 keys 1.06
-// instead of 0.63 ms).  pd_load_sector_cg reads L2, for words that other threads
-// may be changing.
+// waits for its compare-and-swap).
+// pd_load_sector_na finds a line that is in L1 but gives none a place there,
+// which is cheaper where no line is read again (probe 2.77 ms).  It is no use
+// alone: the reads of a small table, or of the hot keys of a skewed probe, then
+// all go to the same few lines of L2 (2^26 rows against 100 build rows 2.24 ms,
+// 0.54 with places; against 10^6 with half of the rows on 20 keys 1.06 and 0.63).
+// One read in a few with a place brings such lines in and leaves most of L1 to
+// what else is read; the callers choose how many.
+// pd_load_sector_cg reads L2, for words that other threads may be changing.
 __device__ __forceinline__ void pd_load_sector(const void *p, ulonglong2 *a, ulonglong2 *b) {
   asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(a->x), "=l"(a->y), "=l"(b->x), "=l"(b->y) : "l"(p));
+}
+__device__ __forceinline__ void pd_load_sector_na(const void *p, ulonglong2 *a, ulonglong2 *b) {
+  asm volatile("ld.global.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
                : "=l"(a->x), "=l"(a->y), "=l"(b->x), "=l"(b->y) : "l"(p));
 }
 __device__ __forceinline__ void pd_load_sector_cg(const void *p, ulonglong2 *a, ulonglong2 *b) {

@@ -282,7 +282,11 @@ __device__ __forceinline__ void hj_probe_tile(const JoinParams &p, uint64_t row0
 #pragma unroll
       for (int i = 0; i < HJ_BATCH; ++i) {
         if (active[i]) {
-          pd_load_sector(p.table + 4 * (uint64_t)g[i], &glo[i], &ghi[i]);
+          // one row of a thread's HJ_ITEMS gives its line a place in L1 (2^26
+          // uniform rows against 60,000 build rows 577 us, all rows 590, none
+          // 571; half of them on 20 of 10^6 keys 620, 628, 1058)
+          if (b + i == 0) pd_load_sector(p.table + 4 * (uint64_t)g[i], &glo[i], &ghi[i]);
+          else pd_load_sector_na(p.table + 4 * (uint64_t)g[i], &glo[i], &ghi[i]);
           any = true;
         }
       }
@@ -1403,6 +1407,7 @@ struct SjaParams {
   const unsigned long long *table;  // the slots, after the table's 32-byte header
   uint32_t bits;
   const uint32_t *side_count, *dup_flag;
+  uint32_t na_mask;  // turns (of a warp's chains) whose bucket lines get no place in L1
   const uint8_t *flag;
   const int64_t *price;
   const int32_t *discount;
@@ -1437,7 +1442,9 @@ __global__ void __launch_bounds__(SJA_THREADS, PD_SJA_CTAS) k_sja_aggregate(SjaP
   const uint32_t side = *p.side_count;
   const bool no_dup = *p.dup_flag == 0;
   bool bad = false;
+  uint32_t turn = 0;
   auto chain = [&](uint32_t r) {
+    ++turn;
     const uint32_t key = __ldg(p.jkey + r);
     const uint32_t f = p.flag ? __ldg(p.flag + r) : 0u;
     const int64_t price = __ldg(p.price + r);
@@ -1459,7 +1466,8 @@ __global__ void __launch_bounds__(SJA_THREADS, PD_SJA_CTAS) k_sja_aggregate(SjaP
     uint32_t b = bucket_of(key, p.bits);
     for (uint64_t step = 0; step <= gmask; ++step) {
       ulonglong2 lo, hi;
-      pd_load_sector(p.table + 4 * (uint64_t)b, &lo, &hi);
+      if ((turn & p.na_mask) == 0) pd_load_sector(p.table + 4 * (uint64_t)b, &lo, &hi);
+      else pd_load_sector_na(p.table + 4 * (uint64_t)b, &lo, &hi);
       const unsigned long long e[4] = {lo.x, lo.y, hi.x, hi.y};
       bool empty = false, found = false;
 #pragma unroll
@@ -1611,6 +1619,11 @@ extern "C" int pimdal_select_join_aggregate(pimdal_ctx_t *ctx,
   uint32_t bits = 0;
   while ((1ull << bits) < a->table_size) ++bits;
   p.bits = bits;
+  // Tables of up to 128 KB keep all their lines in L1, larger ones those of
+  // every fourth turn (3e7 rows, all selected; places for all, every fourth and
+  // none: 100 build rows 217, 272 and 1057 us, 4e6 rows 287, 279 and 269, and with
+  // 3000 keys, whose sums leave the columns little of L1, 1073, 700 and 545).
+  p.na_mask = bits <= 14 ? 0 : 3;
   p.flag = a->flag;
   p.price = a->price;
   p.discount = a->discount;

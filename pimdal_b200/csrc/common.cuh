@@ -219,7 +219,8 @@ __device__ __forceinline__ uint64_t pd_load_relaxed_u64(const uint64_t *p) {
 // all go to the same few lines of L2 (2^26 rows against 100 build rows 2.24 ms,
 // 0.54 with places; against 10^6 with half of the rows on 20 keys 1.06 and 0.63).
 // One read in a few with a place brings such lines in and leaves most of L1 to
-// what else is read; the callers choose how many.
+// what else is read; the callers choose how many, in straight code or by a
+// value of the moment (pd_load_sector_if: no place where na is not 0).
 // pd_load_sector_cg reads L2, for words that other threads may be changing.
 __device__ __forceinline__ void pd_load_sector(const void *p, ulonglong2 *a, ulonglong2 *b) {
   asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
@@ -228,6 +229,13 @@ __device__ __forceinline__ void pd_load_sector(const void *p, ulonglong2 *a, ulo
 __device__ __forceinline__ void pd_load_sector_na(const void *p, ulonglong2 *a, ulonglong2 *b) {
   asm volatile("ld.global.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
                : "=l"(a->x), "=l"(a->y), "=l"(b->x), "=l"(b->y) : "l"(p));
+}
+__device__ __forceinline__ void pd_load_sector_if(const void *p, uint32_t na, ulonglong2 *a, ulonglong2 *b) {
+  asm volatile(
+      "{\n\t.reg .pred place;\n\tsetp.eq.u32 place, %5, 0;\n\t"
+      "@place ld.global.v4.b64 {%0, %1, %2, %3}, [%4];\n\t"
+      "@!place ld.global.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&l"(a->x), "=&l"(a->y), "=&l"(b->x), "=&l"(b->y) : "l"(p), "r"(na));
 }
 __device__ __forceinline__ void pd_load_sector_cg(const void *p, ulonglong2 *a, ulonglong2 *b) {
   asm volatile("ld.global.cg.v4.b64 {%0, %1, %2, %3}, [%4];"

@@ -1466,8 +1466,7 @@ __global__ void __launch_bounds__(SJA_THREADS, PD_SJA_CTAS) k_sja_aggregate(SjaP
     uint32_t b = bucket_of(key, p.bits);
     for (uint64_t step = 0; step <= gmask; ++step) {
       ulonglong2 lo, hi;
-      if ((turn & p.na_mask) == 0) pd_load_sector(p.table + 4 * (uint64_t)b, &lo, &hi);
-      else pd_load_sector_na(p.table + 4 * (uint64_t)b, &lo, &hi);
+      pd_load_sector_if(p.table + 4 * (uint64_t)b, turn & p.na_mask, &lo, &hi);
       const unsigned long long e[4] = {lo.x, lo.y, hi.x, hi.y};
       bool empty = false, found = false;
 #pragma unroll
@@ -1621,8 +1620,8 @@ extern "C" int pimdal_select_join_aggregate(pimdal_ctx_t *ctx,
   p.bits = bits;
   // Tables of up to 128 KB keep all their lines in L1, larger ones those of
   // every fourth turn (3e7 rows, all selected; places for all, every fourth and
-  // none: 100 build rows 217, 272 and 1057 us, 4e6 rows 287, 279 and 269, and with
-  // 3000 keys, whose sums leave the columns little of L1, 1073, 700 and 545).
+  // none: 100 build rows 219, 272 and 1057 us, 4e6 rows 282, 275 and 268, and with
+  // 3000 keys, whose sums leave the columns little of L1, 1081, 703 and 537).
   p.na_mask = bits <= 14 ? 0 : 3;
   p.flag = a->flag;
   p.price = a->price;

@@ -1619,10 +1619,15 @@ extern "C" int pimdal_select_join_aggregate(pimdal_ctx_t *ctx,
   while ((1ull << bits) < a->table_size) ++bits;
   p.bits = bits;
   // Tables of up to 128 KB keep all their lines in L1, larger ones those of
-  // every fourth turn (3e7 rows, all selected; places for all, every fourth and
-  // none: 100 build rows 219, 272 and 1057 us, 4e6 rows 282, 275 and 268, and with
-  // 3000 keys, whose sums leave the columns little of L1, 1081, 703 and 537).
-  p.na_mask = bits <= 14 ? 0 : 3;
+  // every fourth turn (3e7 rows, all selected, us; places for all, every fourth and
+  // none: 100 build rows 219, 272 and 1057, 4e6 rows 282, 275 and 268).  The sums
+  // of key spaces above 2048 leave L1 little, and that to the columns too: there
+  // tables of up to 16 KB keep all, up to 128 KB every fourth and larger ones every
+  // sixteenth (3000 keys; all, every fourth, every sixteenth: 100 build rows 395,
+  // 508 and more, 8000 rows 609, 459 and 441, 4e6 rows 1063, 661 and 576, none 552;
+  // 2000 rows with half of the reads on 20 keys 502, 499 and 592).
+  if (a->key_space <= 2048) p.na_mask = bits <= 14 ? 0 : 3;
+  else p.na_mask = bits <= 11 ? 0 : bits <= 14 ? 3 : 15;
   p.flag = a->flag;
   p.price = a->price;
   p.discount = a->discount;

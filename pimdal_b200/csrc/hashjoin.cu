@@ -1134,12 +1134,15 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
   const unsigned clear_grid = (unsigned)std::min<uint64_t>(pd_ceil_div(1ull << l.bits, 512), ctx->sm_count * 8ull);
   const unsigned build_grid = ctx->sm_count * 8;
   const int pgrid = probe_grid(ctx);
-  // Early launches pay where launches count (us with and without: 1e6 probe rows
-  // 32.9 and 36.6, 2^24 rows 235 and 245, 2^25 rows 761 and 767; 2^26 rows the
-  // same); in a larger join the next kernel's waiting CTAs cost more than its
-  // launch (2^28 rows 5.69 and 5.54 ms).  A build or a probe by itself and the
-  // partition passes lose nothing at any size and are always launched early.
-  const bool early = a->size_probe < (1u << 26);
+  // An SM changes its split between L1 and shared memory only while it is idle.
+  // Launched early behind a partition pass, which takes up to 222 KB of shared
+  // memory, the clear kept the SMs busy, and the build and the probe, launched
+  // early behind it, ran with what L1 that pass had left (8e6 x 2^24 rows in 64
+  // partitions 592 -> 889 us, 2^25 x 2^28 rows 5.49 -> 5.62 ms).  So the clear is an
+  // ordinary launch, but for short joins without partitions, where each launch
+  // counts (1e6 probe rows, us: none early 36.6, all three 32.9); the build and
+  // the probe are always early (1e6 x 2^24 rows 206 -> 202 us).
+  const bool early = !l.part_bits && a->size_probe < (1u << 24);
   // One table of 2^bits slots, one build and one probe launch over the
   // (partitioned) rows.  A key's home bucket is the top bits of the same hash
   // whose top part_bits chose its partition, so the rows of partition q touch
@@ -1151,11 +1154,11 @@ extern "C" int pimdal_hash_join(pimdal_ctx_t *ctx, const pimdal_hash_join_argume
   }
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_BUILD, s);
-    PD_CHECK_CUDA(pd_launch_early(early, k_hj_build, build_grid, 256, 0, s, 1, p));
+    PD_CHECK_CUDA(pd_launch(k_hj_build, build_grid, 256, 0, s, 1, p));
   }
   {
     pd_launch_scope sc(ctx, PIMDAL_KERNEL_HJ_PROBE, s);
-    PD_CHECK_CUDA(pd_launch_early(early, k_hj_probe, pgrid, HJ_THREADS, 0, s, 1, p));
+    PD_CHECK_CUDA(pd_launch(k_hj_probe, pgrid, HJ_THREADS, 0, s, 1, p));
   }
   return pd_launch_status(ctx);
 }

@@ -1,0 +1,35 @@
+"""Kernels that are launched early leave the SMs to run as they would behind an
+ordinary launch: joins behind partition passes, merges behind sorts."""
+import pytest
+import torch
+
+from pimdal_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def ms(ctx, run):
+    best = 1e9
+    for _ in range(6):
+        a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+        a.record()
+        run()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b))
+    ctx.sync()
+    return best
+
+
+def test_hash_join_of_64_partitions(ctx):
+    """1.5 times the time of 16 partitions when the clear was launched early."""
+    nb, n = 8_000_000, 1 << 24
+    build = torch.randperm(2 * nb, dtype=torch.int32, device="cuda")[:nb]
+    probe = torch.randint(0, 2 * nb, (n,), dtype=torch.int32, device="cuda")
+    pay, row = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+
+    def join(bits):
+        return ms(ctx, lambda: ops.hash_join(ctx, build, build, probe, partition_bits=bits, out_payload=pay,
+                                             out_row=row))
+
+    assert join(6) < 1.2 * join(4)

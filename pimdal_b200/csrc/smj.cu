@@ -73,7 +73,11 @@ __device__ __forceinline__ uint64_t gsearch(const uint32_t *key, uint64_t lo, ui
 }
 
 __global__ void __launch_bounds__(256) k_smj_bounds(MergeParams p) {
-  pd_grid_dep();
+  // The merge comes onto the SMs only when the sorts are complete: it has one CTA
+  // per tile, and on SMs that a sort's last pass had half filled its CTAs lay
+  // in heaps (3e5 x 3e5 rows with each key 4 times 208 us against 129).
+  pd_grid_wait();
+  pd_grid_trigger();
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0) *p.claim = 0;  // the merge's tile counter
   if (t >= p.tiles) return;
